@@ -288,21 +288,25 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const u
             }
 }
 
-// gvdbCalcSubcellPos (P:677-694)
+// gvdbCalcSubcellPos (P:677-694), a thread per subcell of every pool leaf
+// (scpb subcells a leaf, 512 of them in a 32^3 brick).  Bound by its 16 bytes
+// of stores a subcell; a thread per leaf that looped over its subcells left
+// all but a few warps idle (150 bricks of 32^3: 313 us, 48 bricks: 177 us;
+// a thread per subcell: 3 us).
 __global__ void k_sc_pos(const Node *leaves, int64_t n, const uint32_t *mapping, int sc, int scdim, int scpb,
                          int64_t num_sc, int32_t *sc_nid, int32_t *sc_pos) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n * scpb) return;
+    const int64_t i = t / scpb;
+    const int s = (int)(t - i * scpb);
     const Node &nd = leaves[i];
     if (nd.mParent == kUndef64) return;
-    for (int s = 0; s < scpb; s++) {
-        int64_t idx = (int64_t)mapping[i] * scpb + s;
-        if (idx >= num_sc) continue;
-        sc_pos[3 * idx + 0] = nd.mPos[0] + s % scdim * sc;
-        sc_pos[3 * idx + 1] = nd.mPos[1] + (s / scdim) % scdim * sc;
-        sc_pos[3 * idx + 2] = nd.mPos[2] + (s / scdim / scdim) % scdim * sc;
-        sc_nid[idx] = (int32_t)i;
-    }
+    const int64_t idx = (int64_t)mapping[i] * scpb + s;
+    if (idx >= num_sc) return;
+    sc_pos[3 * idx + 0] = nd.mPos[0] + s % scdim * sc;
+    sc_pos[3 * idx + 1] = nd.mPos[1] + (s / scdim) % scdim * sc;
+    sc_pos[3 * idx + 2] = nd.mPos[2] + (s / scdim / scdim) % scdim * sc;
+    sc_nid[idx] = (int32_t)i;
 }
 
 } // namespace
@@ -527,9 +531,9 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
                                                                          v->sc_pnt.as<float>(), status);
         }
     }
-    k_sc_pos<<<grid_for(nmap, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, v->sc_map.as<uint32_t>(), sc, scdim,
-                                                            scpb, num_sc, v->sc_nid.as<int32_t>(),
-                                                            v->sc_pos.as<int32_t>());
+    k_sc_pos<<<grid_for(nmap * scpb, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, v->sc_map.as<uint32_t>(), sc,
+                                                                   scdim, scpb, num_sc, v->sc_nid.as<int32_t>(),
+                                                                   v->sc_pos.as<int32_t>());
     GV_CUDA(v, cudaGetLastError());
     cudaFreeAsync(status, s);
     return GVDB2_OK;

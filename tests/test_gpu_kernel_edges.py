@@ -1,0 +1,26 @@
+"""GPU parity at the sizes where single kernels can go wrong: the ends of
+their tiles, remainders, the smallest and the largest of their range."""
+import numpy as np
+import pytest
+
+from _helpers import make_oracle
+from test_gpu_topology import gpu_volume
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sc,cfg", [(2, (3, 3, 3, 3, 3)), (8, (3, 3, 3, 3, 3)), (4, (3, 3, 3, 3, 5)), (16, (3, 3, 3, 3, 5))])
+def test_subcell_table(gvdb2_mod, oracle_mod, sc, cfg):
+    """Every subcell's node and corner, for 1, 8, 64 and 512 subcells a brick, against the oracle (exact)."""
+    rng = np.random.default_rng(20)
+    pts = rng.uniform(70.0, 170.0, (3001, 3)).astype(np.float32)
+    o = make_oracle(oracle_mod, cfg)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.insert_points_subcell(sc, pts, 2.0)
+    cnt, nid, pos = o.subcells()
+    v = gpu_volume(gvdb2_mod, pts, cfg)
+    v.RebuildTopology(len(pts), 2.0)
+    v.InsertPointsSubcell(sc, len(pts), 2.0)
+    g = v.subcells(len(cnt))
+    for a, b in zip(g, (cnt, nid, pos)):
+        assert np.array_equal(a, b)
