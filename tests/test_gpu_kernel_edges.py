@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from _helpers import make_oracle
-from test_gpu_topology import gpu_volume
+from test_gpu_topology import compare_topology, gpu_volume
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +24,19 @@ def test_subcell_table(gvdb2_mod, oracle_mod, sc, cfg):
     g = v.subcells(len(cnt))
     for a, b in zip(g, (cnt, nid, pos)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("lo,hi", [
+    ((70.0, 70.0, 70.0), (73.0, 73.0, 73.0)),       # a grid of less than one 32-bit word
+    ((68.0, 70.0, 66.0), (69.0, 71.0, 320.0)),      # one brick thick, several parents long
+    ((61.0, 3.0, 509.0), (67.0, 260.0, 900.0)),     # parents that start inside the grid, two levels of them
+])
+def test_parent_levels(gvdb2_mod, oracle_mod, lo, hi):
+    """Node pools and child lists of small and thin brick grids, against the oracle (exact)."""
+    rng = np.random.default_rng(21)
+    pts = rng.uniform(lo, hi, (400, 3)).astype(np.float32)
+    o = make_oracle(oracle_mod)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    v = gpu_volume(gvdb2_mod, pts)
+    v.RebuildTopology(len(pts), 2.0)
+    compare_topology(v, o)
