@@ -212,8 +212,37 @@ __device__ __forceinline__ bool in_range(const SplatLimits &L, int64_t i, int64_
 }
 constexpr uint32_t kSlicePts = 4096;
 // cell_cnt entries: huge, heavy, light cells; dense cells, dense work
-// items (slices), dense cells of more than one slice
-constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntWords = 8;
+// items (slices), dense cells of more than one slice, cells listed for
+// k_scatter_cells, dense cells listed for k_scatter_rows
+constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntOwner = 6,
+              kCntRows = 7, kCntWords = 8;
+// Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic): 16.7M
+// points in cells of 1,024 on average, 4 channels, 1.22 + 0.13 ms (its sort)
+// against 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162
+// short units (a 300,000-point blob's cells of 512 to 700: 48 us against 20), more
+// make a cell its launch's tail.
+#ifndef GVDB2_ROWS_MIN
+#define GVDB2_ROWS_MIN 768
+#endif
+#ifndef GVDB2_ROWS_MAX
+#define GVDB2_ROWS_MAX 2048
+#endif
+constexpr int kRowsMin = GVDB2_ROWS_MIN, kRowsMax = GVDB2_ROWS_MAX;
+static_assert(kRowsMax <= 65535, "16-bit positions in a cell");
+// Most points of a cell that k_scatter_light serves, and (cubic) of its face
+// neighbours, dense cells not counted.  Scatter passes at 32, 64 and 96 points:
+// one channel, 612k cells of 9 points on average 1.49, 1.42, 1.39 ms; three
+// channels, a 300,000-point blob 146, 141, 138 us; four channels, 634k cells of 26
+// points 4.98, 4.86, 4.78 ms.  Without the rule on neighbours the cells around a
+// block of 256 points a cell (four channels) cost 35 us of 795; with it 18 us.
+#ifndef GVDB2_LIGHT_OWN
+#define GVDB2_LIGHT_OWN 96
+#endif
+#ifndef GVDB2_HEAVY_FACE
+#define GVDB2_HEAVY_FACE 192
+#endif
+constexpr int32_t kPartListed = -2; // a cell's partial slot when it is listed for k_scatter_cells
+constexpr int kLightOwn = GVDB2_LIGHT_OWN, kHeavyFace = GVDB2_HEAVY_FACE;
 // The i-th huge or heavy cell, or -1 past their end.
 __device__ __forceinline__ int64_t cell_at(int64_t i, const int32_t *list, const uint32_t *cnt, int64_t ncell) {
     const int64_t h = cnt[0];
@@ -283,6 +312,7 @@ struct Taps<GVDB2_KERNEL_TENT1> {
         w[1] = t;
         return (int)b;
     }
+    __device__ __forceinline__ static int eval_fine(float x, float w[2]) { return eval(x, w); }
     __device__ __forceinline__ static int eval_d(float x, float w[2], float dw[2]) {
         int f = eval(x, w);
         dw[0] = -1.0f;
@@ -307,16 +337,35 @@ struct Taps<GVDB2_KERNEL_CUBIC2> {
         w[3] = t * t * t * k6;
         return (int)b - 1;
     }
+    // The same weights with x / 6 from the float nearest to 1/6 and what it lacks.
+    // The first alone is 3e-8 too large, the same way on every axis: most of the
+    // 2.4e-7 by which a cubic splat and gather missed 64 bits.  The splat kernels
+    // whose sums deterministic mode uses keep eval, so that its results stay what
+    // they were bit for bit.
+    __device__ __forceinline__ static float sixth(float x) {
+        constexpr float hi = 1.0f / 6.0f, lo = (float)(1.0 / 6.0 - (double)hi);
+        return fmaf(x, hi, x * lo);
+    }
+    __device__ __forceinline__ static int eval_fine(float x, float w[4]) {
+        float u = x - 0.5f;
+        float b = floorf(u);
+        float t = u - b;
+        float s = 1.0f - t;
+        w[0] = sixth(s * s * s);
+        w[1] = sixth((3.0f * t - 6.0f) * t * t + 4.0f);
+        w[2] = sixth(((-3.0f * t + 3.0f) * t + 3.0f) * t + 1.0f);
+        w[3] = sixth(t * t * t);
+        return (int)b - 1;
+    }
     __device__ __forceinline__ static int eval_d(float x, float w[4], float dw[4]) {
         float u = x - 0.5f;
         float b = floorf(u);
         float t = u - b;
         float s = 1.0f - t;
-        const float k6 = 1.0f / 6.0f;
-        w[0] = s * s * s * k6;
-        w[1] = ((3.0f * t - 6.0f) * t * t + 4.0f) * k6;
-        w[2] = (((-3.0f * t + 3.0f) * t + 3.0f) * t + 1.0f) * k6;
-        w[3] = t * t * t * k6;
+        w[0] = sixth(s * s * s);
+        w[1] = sixth((3.0f * t - 6.0f) * t * t + 4.0f);
+        w[2] = sixth(((-3.0f * t + 3.0f) * t + 3.0f) * t + 1.0f);
+        w[3] = sixth(t * t * t);
         dw[0] = -0.5f * s * s;
         dw[1] = (1.5f * t - 2.0f) * t;
         dw[2] = (-1.5f * t + 1.0f) * t + 0.5f;

@@ -197,7 +197,15 @@ struct Volume {
     // cells whose voxels k_scatter_merge adds partials to (count in the
     // last 16 bytes)
     DevBuf merge_list;
+    // cells of more than kLightOwn points that are not dense
+    DevBuf cell_owner;
     int64_t dense_cap = 0, work_cap = 0, multi_cap = 0, part_acc_cap = 0;
+    // the dense cells that k_scatter_rows takes (cubic): their list and its
+    // capacity, their keys' first positions (the sorted order itself is in
+    // prank) and whether the scatter has sorted them since the binning
+    DevBuf rows_list, row_off;
+    int64_t rows_cap = 0;
+    bool rows_sorted = false;
     // cells that hold points: huge and heavy ones (order of cell_at), light
     // ones and the counts (kCnt*); heavy_grid, light_grid and cell_grid
     // bound the huge+heavy, light and all lists

@@ -150,12 +150,19 @@ __global__ void k_bin_pack_pos(const int32_t *perm, const uint32_t *reg_off, int
 constexpr int64_t kCellCountReadback = 1 << 16; // cells
 
 // Cells of at least `dense_min` points (dense_min > 0) are the scatter's dense
-// cells: each gets a partial slot (part[c], -1 for the other cells),
+// cells: each gets a partial slot (part[c], -1 or kPartListed for the other cells),
 // ceil(k / slice) work items (cell, slice, slices, accumulator slot) and,
 // when that is more than one, an accumulator slot for its integer sums.
-// Cells of at most `light` (<= kLightCell) points are light.
+// With rows_on the dense cells of kRowsMin to kRowsMax points are listed in
+// `rows` instead of the work items.  Cells of at most `light` (<= kLightCell) points are light.  The cells of more
+// than kLightOwn points that are not dense and, for the cubic, those with a face
+// neighbour of more than kHeavyFace (not dense either) are listed in `owner`.  It depends on
+// the cell and its neighbours alone, so that a cloud of a batch gets what a
+// volume of its own gets.
 __global__ void k_cell_list(const uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int32_t *part,
-                            int4 *work, uint32_t *cnt, uint32_t dense_min, uint32_t slice, uint32_t light_max) {
+                            int32_t *owner, int32_t *rows, int4 *work, uint32_t *cnt, const int32_t *nbr27, int m,
+                            uint32_t dense_min,
+                            uint32_t slice, uint32_t light_max, bool cubic, bool rows_on) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k = c < ncell ? off[c + 1] - off[c] : 0u;
     const int cls = k == 0 ? -1 : (k > kHeavyCell ? kCntHuge : (k > light_max ? kCntHeavy : kCntLight));
@@ -169,8 +176,36 @@ __global__ void k_cell_list(const uint32_t *off, int64_t ncell, int32_t *list, i
     const unsigned dn = __ballot_sync(0xffffffffu, dense);
     int32_t slot = -1;
     if (dense) slot = (int32_t)warp_agg_inc(cnt, (uint32_t)kCntDense, dn);
-    if (c < ncell) part[c] = slot;
-    if (dense) {
+    // many points of its own, or (cubic: the stencils of 3/8 of a cell's points
+    // reach past a face, of the tent's 1/8) of a face neighbour's
+    bool own = !dense && k > (uint32_t)kLightOwn;
+    if (cubic && !dense && !own && c < ncell) {
+        int64_t slot;
+        int cc[3];
+        cell_coords(c, m, m * m * m, slot, cc[0], cc[1], cc[2]);
+        for (int f = 0; f < 6 && !own; f++) {
+            int nc[3] = {cc[0], cc[1], cc[2]};
+            const int a = f >> 1, d = (f & 1) * 2 - 1;
+            nc[a] += d;
+            int64_t ns = slot;
+            if (nc[a] < 0 || nc[a] >= m) {
+                const int step[3] = {1, 3, 9};
+                ns = nbr27[slot * 27 + 13 + d * step[a]];
+                nc[a] -= d * m;
+            }
+            if (ns < 0) continue;
+            const int64_t n = ns * m * m * m + (nc[2] * m + nc[1]) * m + nc[0];
+            const uint32_t kn = off[n + 1] - off[n];
+            own = kn > (uint32_t)kHeavyFace && !(dense_min > 0 && kn >= dense_min);
+        }
+    }
+    if (c < ncell) part[c] = own ? kPartListed : slot;
+    const unsigned on = __ballot_sync(0xffffffffu, own);
+    if (own) owner[warp_agg_inc(cnt, (uint32_t)kCntOwner, on)] = (int32_t)c;
+    const bool row = rows_on && dense && k >= (uint32_t)kRowsMin && k <= (uint32_t)kRowsMax;
+    const unsigned rn = __ballot_sync(0xffffffffu, row);
+    if (row) rows[warp_agg_inc(cnt, (uint32_t)kCntRows, rn)] = (int32_t)c;
+    if (dense && !row) {
         const uint32_t ns = (k + slice - 1) / slice;
         const uint32_t first = atomicAdd(cnt + kCntWork, ns);
         const int32_t acc = ns > 1 ? (int32_t)atomicAdd(cnt + kCntMulti, 1u) : -1;
@@ -406,12 +441,19 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     GV_CUDA(v, v->cell_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     GV_CUDA(v, v->cell_light.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     GV_CUDA(v, v->cell_part.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
+    GV_CUDA(v, v->cell_owner.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     // bounds from the point count: at most n / dense dense cells, and each
     // slice beyond a cell's first holds `slice` of its points
+    const bool cubic = kernel == GVDB2_KERNEL_CUBIC2;
+    // deterministic mode keeps the fixed-point sums, which no order changes
+    const bool rows = cubic && !v->deterministic;
     const int64_t dmin = v->tune_dense, sl = v->tune_slice;
     v->dense_cap = dmin > 0 ? std::min<int64_t>(nbins, n / dmin) : 0;
+    v->rows_cap = rows ? std::min<int64_t>(v->dense_cap, n / kRowsMin) : 0;
+    v->rows_sorted = false;
     v->work_cap = dmin > 0 ? v->dense_cap + n / sl : 0;
     v->multi_cap = std::min<int64_t>(v->dense_cap, n / (sl + 1));
+    GV_CUDA(v, v->rows_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(v->rows_cap, 1), s));
     GV_CUDA(v, v->part_work.ensure(sizeof(int4) * (size_t)std::max<int64_t>(v->work_cap, 1), s));
     GV_CUDA(v, v->cell_cnt.ensure(sizeof(uint32_t) * kCntWords, s));
     GV_CUDA(v, cudaMemsetAsync(v->cell_cnt.p, 0, sizeof(uint32_t) * kCntWords, s));
@@ -420,9 +462,10 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     if (nbins > 0) {
         const int g = grid_for(nbins, 256, 1ll << 31);
         k_cell_list<<<g, 256, 0, s>>>(v->bin_off.as<uint32_t>(), nbins, v->cell_list.as<int32_t>(),
-                                      v->cell_light.as<int32_t>(), v->cell_part.as<int32_t>(),
-                                      v->part_work.as<int4>(), v->cell_cnt.as<uint32_t>(), (uint32_t)v->tune_dense,
-                                      (uint32_t)v->tune_slice, (uint32_t)v->tune_light);
+                                      v->cell_light.as<int32_t>(), v->cell_part.as<int32_t>(), v->cell_owner.as<int32_t>(),
+                                      v->rows_list.as<int32_t>(), v->part_work.as<int4>(), v->cell_cnt.as<uint32_t>(),
+                                      v->nbr27.as<int32_t>(), m, (uint32_t)dmin, (uint32_t)v->tune_slice, (uint32_t)v->tune_light,
+                                      cubic, rows);
         GV_CUDA(v, cudaGetLastError());
         v->cell_grid = v->heavy_grid = v->light_grid = nbins;
         if (nbins > kCellCountReadback) {
@@ -435,6 +478,7 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
             v->light_grid = cw[kCntLight];
             v->cell_grid = v->heavy_grid + v->light_grid;
             v->dense_cap = cw[kCntDense];
+            v->rows_cap = cw[kCntRows];
             v->work_cap = cw[kCntWork];
             v->multi_cap = cw[kCntMulti];
         }

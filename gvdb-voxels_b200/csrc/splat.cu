@@ -228,6 +228,8 @@ struct SplatArgs {
     // cells with a dense cell among their 27 (k_scatter_cells lists them)
     int32_t *merge_list;
     uint32_t *merge_cnt;
+    // the cells of k_scatter_cells: more than kLightOwn points, not dense
+    const int32_t *owner_list;
 };
 
 
@@ -583,6 +585,664 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
     if (threadIdx.x == 0) S.part_done[item.w] = 0;
 }
 
+// A voxel's channels side by side in a shared-memory tile: one access per tap
+// serves every channel.
+template <int NCH> struct GVec { using T = float4; };
+template <> struct GVec<1> { using T = float; };
+template <> struct GVec<2> { using T = float2; };
+template <int NCH>
+__device__ __forceinline__ void gvec_put(typename GVec<NCH>::T &v, const float (&g)[NCH]) {
+    if constexpr (NCH == 1) v = g[0];
+    else if constexpr (NCH == 2) v = make_float2(g[0], g[1]);
+    else if constexpr (NCH == 3) v = make_float4(g[0], g[1], g[2], 0.0f);
+    else v = make_float4(g[0], g[1], g[2], g[3]);
+}
+template <int NCH>
+__device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *g) {
+    if constexpr (NCH == 1) g[0] = v;
+    else if constexpr (NCH == 2) g[0] = v.x, g[1] = v.y;
+    else {
+        g[0] = v.x, g[1] = v.y, g[2] = v.z;
+        if constexpr (NCH == 4) g[3] = v.w;
+    }
+}
+
+// ---- dense cells, cubic B-spline: sums in registers, row by row -----------
+//
+// The partial of a dense cell of at most kRowsMax points, without atomics.  The
+// points are sorted by their first tap (k_sort_rows) into units: half of the
+// first rows (y0 in [0, 4] or [5, 8]) and one first plane z0 in [0, 8], each in
+// order of the first column x0.  A warp per half takes its units in order of
+// z0: lane (y, z) holds target row y of the half's 8 and target plane z0 + z,
+// and keeps the 4 columns a stencil covers in registers, a window that moves
+// along x; a column that the window leaves is added to the half's planes in
+// shared memory, which hold 5 planes in turn.  After plane z0's last unit its
+// rows, the two halves' sums together, go to the partial.
+//
+// Per point and channel pair a lane adds 4 products (packed FMAs), half of
+// them zero (4 of the 8 rows): bound by instruction issue and by the latency
+// of the records' reads (43% of issue slots, 14 warps an SM: shared memory for
+// 24 KB a cell).  The fixed-point atomics of k_scatter_part, two per tap and
+// channel, are bound by the shared-memory atomic rate, 30 of 32 lanes a cycle.
+//
+// Sums are float, at most some 20 terms in a register window, then up to 8
+// such sums per voxel.
+constexpr int kRowKeys = 2 * 9 * 9; // (half, z0, x0)
+constexpr int kRowOff = kRowKeys + 2;
+constexpr int kSortThreads = 192, kSortWarps = kSortThreads / 32;
+static_assert(kSortThreads >= kRowKeys, "a thread per key");
+
+__device__ __forceinline__ int row_key(int fx, int fy, int fz) {
+    return ((fy >= 5 ? 9 : 0) + fz) * 9 + fx;
+}
+
+// Sorts the points of each listed cell by row_key, points of a key in bin
+// order: order[beg + i] is the bin-order entry of the cell's i-th point in sorted
+// order, row_off[slot] the keys' first positions.  A CTA per cell, each warp a
+// contiguous share of its points.
+__global__ void __launch_bounds__(kSortThreads) k_sort_rows(SplatArgs S, const int32_t *list, int32_t *order,
+                                                            uint16_t *row_off) {
+    using T = Taps<GVDB2_KERNEL_CUBIC2>;
+    constexpr int H = T::N / 2;
+    __shared__ uint32_t hist[kSortWarps][kRowKeys];
+    __shared__ uint32_t wsum[kSortWarps];
+    if (blockIdx.x >= S.cell_cnt[kCntRows]) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t cell = list[blockIdx.x];
+    if (!in_range(S.lim, cell, S.ncell, 30)) return; // the same for the whole CTA
+    const int32_t pslot = S.cell_part[cell];
+    const uint32_t beg = S.bin_off[cell], R = S.bin_off[cell + 1] - beg;
+    if (!in_range(S.lim, pslot, S.dense_cap, 31) || !in_range(S.lim, (int64_t)beg + R - 1, S.lim.nentry, 32)) return;
+    int64_t slot;
+    int cx, cy, cz;
+    cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
+    const int32_t leaf = S.slot_leaf[slot];
+    if (!in_range(S.lim, leaf, S.lim.npool, 33)) return;
+    const Node &nd = S.leaves[leaf];
+    const int ox = nd.mPos[0] + kCell * cx - H, oy = nd.mPos[1] + kCell * cy - H, oz = nd.mPos[2] + kCell * cz - H;
+    for (int i = threadIdx.x; i < kSortWarps * kRowKeys; i += kSortThreads) (&hist[0][0])[i] = 0;
+    __syncthreads();
+    auto key_of = [&](uint32_t j) {
+        const float4 q = S.bin_pos[j];
+        const int32_t cloud = __float_as_int(q.w);
+        int3 o = make_int3(0, 0, 0);
+        if (cloud >= 0 && in_range(S.lim, cloud, S.lim.ncloud, 34))
+            o = make_int3(S.pos.origin[3 * cloud], S.pos.origin[3 * cloud + 1], S.pos.origin[3 * cloud + 2]);
+        const int fx = (int)floorf(q.x - 0.5f) - T::LO + o.x - ox, fy = (int)floorf(q.y - 0.5f) - T::LO + o.y - oy,
+                  fz = (int)floorf(q.z - 0.5f) - T::LO + o.z - oz;
+        return row_key(min(max(fx, 0), 8), min(max(fy, 0), 8), min(max(fz, 0), 8));
+    };
+    const uint32_t share = (R + 32 * kSortWarps - 1) / (32 * kSortWarps) * 32;
+    const uint32_t s0 = min(R, warp * share), s1 = min(R, s0 + share);
+    for (uint32_t j = s0 + lane; j < s1; j += 32) atomicAdd(&hist[warp][key_of(beg + j)], 1u);
+    __syncthreads();
+    { // each key's first position, and each warp's in it
+        const int k = threadIdx.x;
+        uint32_t n = 0;
+        if (k < kRowKeys)
+            for (int w = 0; w < kSortWarps; w++) n += hist[w][k];
+        uint32_t inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        uint32_t run = inc - n;
+        for (int w = 0; w < warp; w++) run += wsum[w];
+        if (k <= kRowKeys) row_off[(int64_t)pslot * kRowOff + k] = (uint16_t)run; // key kRowKeys: all R
+        if (k < kRowKeys)
+            for (int w = 0; w < kSortWarps; w++) {
+                const uint32_t c = hist[w][k];
+                hist[w][k] = run;
+                run += c;
+            }
+    }
+    __syncthreads();
+    for (uint32_t j0 = s0; j0 < s1; j0 += 32) { // in order: stable
+        const uint32_t j = j0 + lane;
+        const bool ok = j < s1;
+        const int k = ok ? key_of(beg + j) : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, k);
+        const uint32_t at = ok ? hist[warp][k] + __popc(peers & lanemask_lt()) : 0u;
+        __syncwarp();
+        if (ok && lane == __ffs(peers) - 1) hist[warp][k] += __popc(peers);
+        __syncwarp();
+        if (ok) order[beg + at] = (int32_t)(beg + j);
+    }
+}
+
+// Position in a cubic partial of extended-tile voxel z * 144 + y * 12 + x.
+struct PartPos {
+    uint16_t pos[ExtTile<GVDB2_KERNEL_CUBIC2>::E3];
+    constexpr PartPos() : pos() {
+        using X = ExtTile<GVDB2_KERNEL_CUBIC2>;
+        for (int z = 0; z < X::E; z++)
+            for (int y = 0; y < X::E; y++)
+                for (int x = 0; x < X::E; x++) pos[(z * X::E + y) * X::E + x] = (uint16_t)X::part_index(x, y, z);
+    }
+};
+__device__ constexpr PartPos kPartPos{};
+
+constexpr int kRowRec = 28; // floats a record: x weights twice each, 8 y weights, z weights, amounts, padding
+template <int NCH>
+struct RowSmem {
+    // [half][plane in turn][row][column]: the odd row stride and the plane stride
+    // of 8 modulo 32 words put a flush's 32 values in different banks
+    typename GVec<NCH>::T plane[2][5][8][13];
+    float rec[2][32][kRowRec];
+    uint16_t off[kRowOff];
+};
+
+template <int NCH>
+__global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t *list, const int32_t *order,
+                                                     const uint16_t *row_off) {
+    using T = Taps<GVDB2_KERNEL_CUBIC2>;
+    using X = ExtTile<GVDB2_KERNEL_CUBIC2>;
+    using V = typename GVec<NCH>::T;
+    constexpr int NP = (NCH + 1) / 2; // channel pairs (one channel: its value twice is not needed, .x only)
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    RowSmem<NCH> &M = *reinterpret_cast<RowSmem<NCH> *>(row_smem);
+    if (blockIdx.x >= S.cell_cnt[kCntRows]) return;
+    const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
+    const int64_t cell = list[blockIdx.x];
+    if (!in_range(S.lim, cell, S.ncell, 35)) return; // the same for the whole CTA
+    const int32_t pslot = S.cell_part[cell];
+    const uint32_t beg = S.bin_off[cell], R = S.bin_off[cell + 1] - beg;
+    if (!in_range(S.lim, pslot, S.dense_cap, 36) || !in_range(S.lim, (int64_t)beg + R - 1, S.lim.nentry, 37)) return;
+    int64_t slot;
+    int cx, cy, cz;
+    cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
+    const int32_t leaf = S.slot_leaf[slot];
+    if (!in_range(S.lim, leaf, S.lim.npool, 38)) return;
+    const Node &nd = S.leaves[leaf];
+    const int ox = nd.mPos[0] + kCell * cx - X::H, oy = nd.mPos[1] + kCell * cy - X::H,
+              oz = nd.mPos[2] + kCell * cz - X::H;
+    for (int i = threadIdx.x; i <= kRowKeys; i += 64) M.off[i] = row_off[(int64_t)pslot * kRowOff + i];
+    {
+        float *z = reinterpret_cast<float *>(M.plane);
+        for (int i = threadIdx.x; i < (int)(sizeof(M.plane) / sizeof(float)); i += 64) z[i] = 0.0f;
+    }
+    __syncthreads();
+    const int ty = lane & 7, tz = lane >> 3;
+    float *dst = S.part + (int64_t)pslot * NCH * X::E3;
+    // The half's points in sorted order, 32 records at a time, one a lane: the
+    // next 32 points' data are on their way from memory while the current 32 are
+    // added.
+    const uint32_t end = M.off[(half + 1) * 81];
+    float4 next_q, next_am;
+    auto fetch = [&](uint32_t i0) {
+        next_q = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+        next_am = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i0 + lane < end) {
+            const int32_t j = order[beg + i0 + lane];
+            if (in_range(S.lim, j, S.lim.nentry, 39)) {
+                next_q = S.bin_pos[j];
+                next_am = S.bin_amt[j];
+            }
+        }
+    };
+    auto stage = [&](uint32_t i0) { // records of points [i0, i0 + 32), fetched before
+        const float4 q = next_q, am = next_am;
+        fetch(i0 + 32);
+        float *r = M.rec[half][lane];
+        float4 *r4 = reinterpret_cast<float4 *>(r);
+        const int32_t cloud = __float_as_int(q.w);
+        int3 o = make_int3(0, 0, 0);
+        if (cloud >= 0 && in_range(S.lim, cloud, S.lim.ncloud, 40))
+            o = make_int3(S.pos.origin[3 * cloud], S.pos.origin[3 * cloud + 1], S.pos.origin[3 * cloud + 2]);
+        float wx[4], wy[4], wz[4];
+        const int fx = T::eval_fine(q.x, wx) + o.x - ox, fy = T::eval_fine(q.y, wy) + o.y - oy - 5 * half,
+                  fz = T::eval_fine(q.z, wz) + o.z - oz;
+        __syncwarp(); // the records before are read
+        r4[0] = make_float4(wx[0], wx[0], wx[1], wx[1]);
+        r4[1] = make_float4(wx[2], wx[2], wx[3], wx[3]);
+        r4[2] = r4[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+        // a binned point's first taps lie in [0, 8] and its rows in the half;
+        // anything else adds nothing
+        const bool ok = (unsigned)fx <= 8u && (unsigned)fz <= 8u && (unsigned)fy <= 4u;
+        if (ok)
+#pragma unroll
+            for (int k = 0; k < 4; k++) r[8 + fy + k] = wy[k];
+        r4[4] = make_float4(wz[0], wz[1], wz[2], wz[3]);
+        r4[5] = am;
+        __syncwarp();
+    };
+    // the values of a record that the lane takes
+    struct Rec {
+        float4 x01, x23, a;
+        float wyz;
+    };
+    auto load = [&](const float *r) {
+        return Rec{reinterpret_cast<const float4 *>(r)[0], reinterpret_cast<const float4 *>(r)[1],
+                   reinterpret_cast<const float4 *>(r)[5], r[8 + ty] * r[16 + tz]};
+    };
+    uint32_t i = M.off[half * 81], staged = i; // the points below `staged` are in rec
+    fetch(i);
+    int turn = 0; // z0 modulo 5
+    for (int z0 = 0; z0 < X::E; z0++) {
+        if (z0 < 9) {
+            const uint16_t *off = M.off + (half * 9 + z0) * 9;
+            if (off[0] < off[9]) {
+                int t = turn + tz;
+                if (t >= 5) t -= 5;
+                V *row = M.plane[half][t][ty];
+                float2 acc[4][NP];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+#pragma unroll
+                    for (int c = 0; c < NP; c++) acc[k][c] = make_float2(0.0f, 0.0f);
+                auto flush = [&](int x, int k) { // window column k (x modulo 4) to column x of the planes
+                    float g[4] = {0.f, 0.f, 0.f, 0.f};
+                    gvec_get<NCH>(row[x], g);
+                    float sum[NCH];
+#pragma unroll
+                    for (int c = 0; c < NCH; c++) sum[c] = g[c] + ((c & 1) ? acc[k][c / 2].y : acc[k][c / 2].x);
+                    gvec_put<NCH>(row[x], sum);
+#pragma unroll
+                    for (int c = 0; c < NP; c++) acc[k][c] = make_float2(0.0f, 0.0f);
+                };
+                auto add = [&](const Rec &p, int x0) {
+                    const float2 ap[2] = {make_float2(p.a.x, p.a.y), make_float2(p.a.z, p.a.w)};
+                    const float2 w[4] = {make_float2(p.x01.x, p.x01.y), make_float2(p.x01.z, p.x01.w),
+                                         make_float2(p.x23.x, p.x23.y), make_float2(p.x23.z, p.x23.w)};
+#pragma unroll
+                    for (int c = 0; c < NP; c++) {
+                        const float2 t2 = __fmul2_rn(ap[c], make_float2(p.wyz, p.wyz));
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            acc[(x0 + k) & 3][c] = __ffma2_rn(t2, w[k], acc[(x0 + k) & 3][c]);
+                    }
+                };
+#pragma unroll
+                for (int x0 = 0; x0 < 9; x0++) {
+                    const uint32_t e = off[x0 + 1];
+                    while (i < e) {
+                        if (i == staged) {
+                            stage(i);
+                            staged = i + 32;
+                        }
+                        const uint32_t m = min(e, staged);
+                        const float *r = M.rec[half][32 + i - staged];
+                        for (; i + 1 < m; i += 2, r += 2 * kRowRec) { // two at a time: their reads overlap
+                            const Rec p = load(r), q = load(r + kRowRec);
+                            add(p, x0);
+                            add(q, x0);
+                        }
+                        if (i < m) {
+                            add(load(r), x0);
+                            i++;
+                        }
+                    }
+                    // no later point reaches column x0
+                    if (e > off[x0 > 3 ? x0 - 3 : 0]) flush(x0, x0 & 3);
+                }
+#pragma unroll
+                for (int x = 9; x < X::E; x++) flush(x, x & 3);
+            }
+        }
+        __syncthreads(); // both halves are done with plane z0
+        // its rows: 0..7 from half 0, 5..11 from half 1; the planes of the next
+        // first plane are other ones, so it may start meanwhile
+        for (int v = threadIdx.x; v < X::E * X::E; v += 64) {
+            const int y = v / X::E, x = v - y * X::E;
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int ly = y - 5 * h;
+                if ((unsigned)ly < 8u) {
+                    float g[4] = {0.f, 0.f, 0.f, 0.f};
+                    gvec_get<NCH>(M.plane[h][turn][ly][x], g);
+                    const float zero[NCH] = {};
+                    gvec_put<NCH>(M.plane[h][turn][ly][x], zero);
+#pragma unroll
+                    for (int c = 0; c < NCH; c++) sum[c] += g[c];
+                }
+            }
+            const int pos = kPartPos.pos[z0 * X::E * X::E + v];
+#pragma unroll
+            for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] = sum[c];
+        }
+        turn = turn == 4 ? 0 : turn + 1;
+    }
+}
+
+// The order of a chunk's records in the owner-computes kernels: first z tap in
+// [-3, 7], then x group (the stencil reaches the lower half of the cell's
+// columns only, both, the upper half only).
+constexpr int kScBins = 11 * 3;
+template <int N>
+__device__ __forceinline__ int sc_key(int fx, int fz) {
+    const int xg = fx < 5 - N ? 0 : (fx <= 3 ? 1 : 2);
+    return min(max(fz + 3, 0), 10) * 3 + xg; // any index is in range, whatever the point
+}
+
+// ---- owner-computes scatter, cells with few sources ----------------------
+//
+// The same sums as k_scatter_cells below for the cells of at most kLightOwn
+// points (and the dense ones, for their neighbours' points): in sparse volumes
+// most of them, where that kernel's 128 registers and its walks over short runs
+// cost far more than the points do.  One warp per cell adds the sources one after
+// the other, in that kernel's order, to a tile of the cell in shared memory, a
+// lane per two taps (a tap for the tent), so no two lanes of a step touch the
+// same voxel; the tile is then written in whole rows.
+//
+// Bound by the latency of its dependent reads (slot -> neighbour -> region
+// offsets -> points) and by the partial sectors of its writes: 612k cells, 5.5M
+// points, one channel 1.51 ms with the share of k_scatter_cells, 2.52 ms all in
+// k_scatter_cells.
+constexpr int kLightWarps = 4;
+constexpr int kLightList = 128; // sources listed at a time
+
+// The up to 63 runs of perm that reach a cell, in a fixed order: run r is
+// regions [r0, r1) of the neighbour in direction d.  Per axis a neighbour
+// below contributes its upper band (region 2), one above its lower band (0),
+// the cell itself all three; regions are ordered (rz, ry, rx), so bands along
+// x are single regions and bands along z are 9 at once.
+struct SrcRuns {
+    uint8_t d[64], r0[64], r1[64];
+    int n, own; // runs; the cell's own one
+    constexpr SrcRuns() : d(), r0(), r1(), n(0), own(0) {
+        for (int dd = 0; dd < 27; dd++) {
+            const int k = dd;
+            const int dx = k % 3 - 1, dy = k / 3 % 3 - 1, dz = k / 9 - 1;
+            const int rx0 = dx < 0 ? 2 : 0, ry0 = dy < 0 ? 2 : 0, ry1 = dy > 0 ? 0 : 2;
+            const int rz0 = dz < 0 ? 2 : 0, rz1 = dz > 0 ? 0 : 2;
+            if (k == 13) own = n;
+            if (dx == 0 && dy == 0) {
+                put(k, rz0 * 9, dz == 0 ? kRegions : rz0 * 9 + 9);
+            } else if (dx == 0) {
+                for (int rz = rz0; rz <= rz1; rz++) put(k, (rz * 3 + ry0) * 3, (rz * 3 + ry0) * 3 + 3);
+            } else {
+                for (int rz = rz0; rz <= rz1; rz++)
+                    for (int ry = ry0; ry <= ry1; ry++) put(k, (rz * 3 + ry) * 3 + rx0, (rz * 3 + ry) * 3 + rx0 + 1);
+            }
+        }
+    }
+    constexpr void put(int k, int a, int b) {
+        d[n] = (uint8_t)k;
+        r0[n] = (uint8_t)a;
+        r1[n] = (uint8_t)b;
+        n++;
+    }
+};
+__device__ constexpr SrcRuns kSrcRuns{};
+static_assert(SrcRuns{}.n == 63, "63 runs");
+
+struct alignas(16) LightRec {
+    float4 wx, wy, wz, am;
+    int32_t at;   // first tap's tile index, z * 64 + y * 8 + x (may be negative)
+    int32_t pack; // its coordinates + 8, a byte each
+    int32_t pad[2];
+};
+template <int NCH>
+struct LightWarp {
+    typename GVec<NCH>::T tile[512]; // voxel (x, y, z) at light_at(z * 64 + y * 8 + x)
+    LightRec rec[32];
+    uint32_t src[kLightList];
+    uint16_t off[kScBins + 1];
+};
+// Half of the rows have their x halves swapped, so that the taps of a step (4 x 4
+// voxels in planes z and z + 2) that one access serves together fall in
+// different banks wherever the stencil lies: for one channel (32 lanes at a
+// time) by bit 1 of z, for two (16: 4 rows) by bit 1 of y, for more (8: 2 rows)
+// by bit 0 of y.
+template <int NCH>
+__device__ __forceinline__ int light_at(int i) {
+    return i ^ ((i >> (NCH == 1 ? 5 : (NCH == 2 ? 2 : 1))) & 4);
+}
+
+// One cell, by one warp.
+template <int KERNEL, int NCH>
+__device__ __forceinline__ void scatter_light_cell(const SplatArgs &S, LightWarp<NCH> &W, int64_t cell, int lane) {
+    using T = Taps<KERNEL>;
+    using V = typename GVec<NCH>::T;
+    constexpr int N = T::N;
+    if (S.cell_part[cell] == kPartListed) return; // k_scatter_cells's
+    int64_t slot;
+    int cx, cy, cz;
+    cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
+    const int32_t leaf = S.slot_leaf[slot];
+    if (!in_range(S.lim, leaf, S.lim.npool, 24)) return; // the same for the whole warp
+    // lane d < 27: the neighbour cell in direction d, or -1 (none, or dense)
+    int32_t nc = -1, pslot = -1;
+    if (lane < 27) {
+        const int ncx = cx + lane % 3 - 1, ncy = cy + lane / 3 % 3 - 1, ncz = cz + lane / 9 - 1;
+        const int bx = ncx < 0 ? -1 : (ncx >= S.m ? 1 : 0), by = ncy < 0 ? -1 : (ncy >= S.m ? 1 : 0),
+                  bz = ncz < 0 ? -1 : (ncz >= S.m ? 1 : 0);
+        int32_t ns = (bx | by | bz) == 0 ? (int32_t)slot
+                                         : S.nbr27[slot * 27 + (bz + 1) * 9 + (by + 1) * 3 + (bx + 1)];
+        if (ns >= 0 && !in_range(S.lim, ns, S.lim.nslot, 25)) ns = -1;
+        if (ns >= 0) { // cells number less than 2^31 / 27
+            nc = ns * S.m3 + ((ncz - bz * S.m) * S.m + (ncy - by * S.m)) * S.m + (ncx - bx * S.m);
+            pslot = S.cell_part[nc];
+            if (pslot >= 0) nc = -1;
+        }
+    }
+    const bool any_part = __any_sync(0xffffffffu, pslot >= 0);
+    // lane l: runs l and l + 32
+    uint32_t first[2], len[2], total = 0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int r = lane + 32 * k;
+        const int32_t c = __shfl_sync(0xffffffffu, nc, kSrcRuns.d[r]);
+        uint32_t a = 0, b = 0;
+        if (r < 63 && c >= 0) {
+            const uint32_t *ro = S.reg_off + (int64_t)c * kRegions;
+            a = ro[kSrcRuns.r0[r]];
+            b = ro[kSrcRuns.r1[r]];
+            if (b > a && !in_range(S.lim, (int64_t)b - 1, S.lim.nentry, 26)) b = a;
+        }
+        first[k] = a;
+        len[k] = b > a ? b - a : 0;
+    }
+    uint32_t before[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        uint32_t inc = len[k];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        before[k] = total + inc - len[k];
+        total += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    // cells with a dense cell around get its partials from k_scatter_merge;
+    // one without sources of its own is listed as ~cell and left for the
+    // merge to write
+    if (any_part) {
+        if (lane == 0) S.merge_list[atomicAdd(S.merge_cnt, 1u)] = total == 0 ? ~(int32_t)cell : (int32_t)cell;
+        if (total == 0) return;
+    }
+    const int a = S.apron, tl = S.tile;
+    const int64_t out0 = slot * S.tvox + ((int64_t)(kCell * cz + a) * tl + (kCell * cy + a)) * tl + (kCell * cx + a);
+    // row = z * 8 + y of the warp's four rows of write step k
+    auto out_at = [&](int k) {
+        const int row = 4 * k + (lane >> 3);
+        return out0 + ((int64_t)(row >> 3) * tl + (row & 7)) * tl + (lane & 7);
+    };
+    if (total == 0) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            const int64_t o = out_at(k);
+#pragma unroll
+            for (int c = 0; c < NCH; c++) S.chan[c][o] = 0.0f;
+        }
+        return;
+    }
+    const Node &nd = S.leaves[leaf];
+    const int ox = nd.mPos[0] + kCell * cx, oy = nd.mPos[1] + kCell * cy, oz = nd.mPos[2] + kCell * cz;
+    // the lane's first tap: (tx, ty, tz0), and (tx, ty, tz0 + 1) for the cubic
+    const int tx = lane & (N - 1), ty = (lane / N) & (N - 1), tz0 = N == 4 ? (lane >> 4) * 2 : (lane >> 2) & 1;
+    const int lat = tz0 * 64 + ty * 8 + tx, lpack = tx | ty << 8 | tz0 << 16;
+    // Lists sources [w0, w0 + kLightList): the cell's own points (run kOwnRun) by
+    // the whole warp, the other runs a lane each.
+    constexpr int kOwnLane = SrcRuns{}.own & 31, kOwnHalf = SrcRuns{}.own >> 5;
+    const uint32_t own0 = __shfl_sync(0xffffffffu, first[kOwnHalf], kOwnLane);
+    const uint32_t own_b = __shfl_sync(0xffffffffu, before[kOwnHalf], kOwnLane);
+    const uint32_t own_e = own_b + __shfl_sync(0xffffffffu, len[kOwnHalf], kOwnLane);
+    auto list = [&](uint32_t w0) {
+        const uint32_t w1 = min(total, w0 + (uint32_t)kLightList);
+        for (uint32_t t = max(own_b, w0) + lane; t < min(own_e, w1); t += 32) W.src[t - w0] = own0 + (t - own_b);
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            if (k != kOwnHalf || lane != kOwnLane)
+                for (uint32_t t = max(before[k], w0); t < min(before[k] + len[k], w1); t++)
+                    W.src[t - w0] = first[k] + (t - before[k]);
+        __syncwarp();
+    };
+    // A source's point, and its first taps in the cell's frame.
+    struct Src {
+        float4 q;
+        int fx, fy, fz;
+    };
+    auto fetch = [&](uint32_t j) {
+        Src d;
+        d.q = S.bin_pos[j];
+        const int32_t cloud = __float_as_int(d.q.w);
+        int3 o = make_int3(0, 0, 0);
+        if (cloud >= 0 && in_range(S.lim, cloud, S.lim.ncloud, 27))
+            o = make_int3(S.pos.origin[3 * cloud], S.pos.origin[3 * cloud + 1], S.pos.origin[3 * cloud + 2]);
+        d.fx = (int)floorf(d.q.x - 0.5f) - T::LO + o.x - ox;
+        d.fy = (int)floorf(d.q.y - 0.5f) - T::LO + o.y - oy;
+        d.fz = (int)floorf(d.q.z - 0.5f) - T::LO + o.z - oz;
+        return d;
+    };
+    auto build = [&](const Src &d, float4 am, int r) { // record r
+        float wx[N], wy[N], wz[N];
+        T::eval(d.q.x, wx);
+        T::eval(d.q.y, wy);
+        T::eval(d.q.z, wz);
+        LightRec &R = W.rec[r];
+        // the stencil reaches the cell on every axis (true of every source
+        // by construction of the regions); anything else adds nowhere
+        const bool ok = d.fx > -N && d.fx < kCell && d.fy > -N && d.fy < kCell && d.fz > -N && d.fz < kCell;
+        R.at = d.fz * 64 + d.fy * 8 + d.fx;
+        R.pack = ok ? (d.fx + 8) | (d.fy + 8) << 8 | (d.fz + 8) << 16 : 0;
+        R.wx = make_float4(wx[0], wx[1], wx[N - 2], wx[N - 1]);
+        R.wy = make_float4(wy[0], wy[1], wy[N - 2], wy[N - 1]);
+        R.wz = make_float4(wz[0], wz[1], wz[N - 2], wz[N - 1]);
+        R.am = am;
+    };
+    auto add = [&](int cnt) { // records [0, cnt) in order
+        for (int i = 0; i < cnt; i++) {
+            const LightRec &R = W.rec[i];
+            const float wx = reinterpret_cast<const float *>(&R.wx)[tx], wy = reinterpret_cast<const float *>(&R.wy)[ty];
+            const float *wz = reinterpret_cast<const float *>(&R.wz);
+            const float4 am = R.am;
+            const float a4[4] = {am.x * wy, am.y * wy, am.z * wy, am.w * wy};
+#pragma unroll
+            for (int k = 0; k < N / 2; k++) { // the lane's taps
+                const int pack = R.pack + lpack + (k << 16);
+                // every coordinate + 8 in [8, 16): the tap lies in the cell
+                if ((pack & 0x181818) == 0x080808 && (N == 4 || lane < 8)) {
+                    const int at = light_at<NCH>(R.at + lat + 64 * k);
+                    const float w = wz[tz0 + k];
+                    V v = W.tile[at];
+                    float g[4] = {0.f, 0.f, 0.f, 0.f};
+                    gvec_get<NCH>(v, g);
+                    float r[NCH];
+#pragma unroll
+                    for (int c = 0; c < NCH; c++) r[c] = fmaf(a4[c] * w, wx, g[c]);
+                    gvec_put<NCH>(v, r);
+                    W.tile[at] = v;
+                }
+            }
+            __syncwarp();
+        }
+    };
+    {
+        float4 *t4 = reinterpret_cast<float4 *>(W.tile);
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(W.tile) / 512); k++) t4[k * 32 + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    // Chunks of kLightList sources, each in the order of k_scatter_cells: by
+    // (first z tap, x group), sources of a key as they come.  A voxel gets the same
+    // products in the same order there, so the two give the same bits.
+    for (uint32_t w0 = 0; w0 < total; w0 += kLightList) {
+        const int cnt = (int)min((uint32_t)kLightList, total - w0);
+        if (w0 > 0) __syncwarp();
+        list(w0);
+        for (int i = lane; i <= kScBins; i += 32) W.off[i] = 0;
+        __syncwarp();
+        Src d{};
+        int key[kLightList / 32];
+        uint32_t rank[kLightList / 32];
+#pragma unroll
+        for (int r = 0; r < kLightList / 32; r++) {
+            if (32 * r >= cnt) break; // the same for the whole warp
+            const int i = 32 * r + lane;
+            key[r] = -1;
+            if (i < cnt) {
+                const Src e = fetch(W.src[i]);
+                if (r == 0) d = e;
+                key[r] = sc_key<N>(e.fx, e.fz);
+            }
+            const unsigned peers = __match_any_sync(0xffffffffu, key[r]);
+            const uint32_t n = key[r] >= 0 ? W.off[key[r]] : 0u;
+            rank[r] = n + __popc(peers & lanemask_lt());
+            __syncwarp();
+            if (key[r] >= 0 && lane == __ffs(peers) - 1) W.off[key[r]] = (uint16_t)(n + __popc(peers));
+            __syncwarp();
+        }
+        { // the keys' first positions; keys 0..31 a lane each, the last one after them
+            const uint32_t n = W.off[lane];
+            uint32_t inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            __syncwarp();
+            W.off[lane] = (uint16_t)(inc - n);
+            if (lane == 31) W.off[32] = (uint16_t)inc;
+        }
+        __syncwarp();
+        if (cnt <= 32) {
+            if (lane < cnt) build(d, S.bin_amt[W.src[lane]], W.off[key[0]] + rank[0]);
+            __syncwarp();
+            add(cnt);
+            continue;
+        }
+        uint32_t j[kLightList / 32];
+#pragma unroll
+        for (int r = 0; r < kLightList / 32; r++) j[r] = 32 * r + lane < cnt ? W.src[32 * r + lane] : 0u;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kLightList / 32; r++)
+            if (32 * r + lane < cnt) W.src[W.off[key[r]] + rank[r]] = j[r];
+        __syncwarp();
+        for (int s0 = 0; s0 < cnt; s0 += 32) {
+            const int m = min(32, cnt - s0);
+            if (lane < m) {
+                const uint32_t e = W.src[s0 + lane];
+                build(fetch(e), S.bin_amt[e], lane);
+            }
+            __syncwarp();
+            add(m);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        float g[4];
+        gvec_get<NCH>(W.tile[light_at<NCH>(32 * k + lane)], g);
+        const int64_t o = out_at(k);
+#pragma unroll
+        for (int c = 0; c < NCH; c++) S.chan[c][o] = g[c];
+    }
+}
+
+template <int KERNEL, int NCH>
+__global__ void __launch_bounds__(32 * kLightWarps) k_scatter_light(SplatArgs S) {
+    extern __shared__ __align__(16) unsigned char light_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t cell = (int64_t)blockIdx.x * kLightWarps + warp;
+    if (cell < S.ncell)
+        scatter_light_cell<KERNEL, NCH>(S, reinterpret_cast<LightWarp<NCH> *>(light_smem)[warp], cell, lane);
+}
+
 // ---- owner-computes scatter --------------------------------------------
 //
 // One warp per cell (an 8^3 block of a brick; the brick itself for 8^3
@@ -622,7 +1282,6 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
 #endif
 constexpr int kScWarps = 4;                    // cells per CTA
 constexpr int kScCap = GVDB2_SC_CAP;           // records per chunk
-constexpr int kScBins = 11 * 3;                // (first z tap + 3, x group)
 
 struct ScChunk {
     // x weights on the cell's voxel columns 0..7: half q (columns 4q..4q+3)
@@ -806,17 +1465,11 @@ __device__ __forceinline__ void sc_accumulate_cp(const ScChunk &C, float2 (&acc)
 // Channel pairs for 2 to 4 channels, x pairs for one channel.
 template <int NCH> struct ScLayout { static constexpr bool kChPairs = GVDB2_SC_CHPAIR && NCH > 1; };
 
-// kScWarps cells per CTA, a warp per cell.
+// One cell, by one warp.
 template <int KERNEL, int NCH>
-__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_cells(SplatArgs S) {
+__device__ __forceinline__ void scatter_cell(const SplatArgs &S, ScChunk &C, int64_t cell, int lane) {
     using T = Taps<KERNEL>;
-    using X = ExtTile<KERNEL>;
     constexpr int N = T::N;
-    extern __shared__ __align__(16) unsigned char sc_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    ScChunk &C = reinterpret_cast<ScChunk *>(sc_smem)[warp];
-    const int64_t cell = (int64_t)blockIdx.x * kScWarps + warp;
-    if (cell >= S.ncell) return;
     int64_t slot;
     int cx, cy, cz;
     cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
@@ -889,7 +1542,8 @@ __global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_
             C.run_first[first + k] = before;
             before += runs[k].y - runs[k].x;
         }
-    const bool any_part = __any_sync(0xffffffffu, pslot >= 0);
+    // a cell with a dense cell around gets its partials from k_scatter_merge
+    if (__any_sync(0xffffffffu, pslot >= 0) && lane == 0) S.merge_list[atomicAdd(S.merge_cnt, 1u)] = (int32_t)cell;
     __syncwarp();
 
     const int y = lane & 7, q = (lane >> 3) & 1, h = lane >> 4;
@@ -981,8 +1635,7 @@ __global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_
             for (int t = 0; t < N; t++) zz4[t] = wzt[t];
             C.wz[r] = make_float4(zz4[0], zz4[1], zz4[2], zz4[3]);
             C.am[r] = make_float4(d.a4[0], d.a4[1], d.a4[2], d.a4[3]);
-            const int xg = fx < 5 - N ? 0 : (fx <= 3 ? 1 : 2); // lower half only, both, upper only
-            C.key[r] = (uint16_t)((fz + 3) * 3 + xg);
+            C.key[r] = (uint16_t)sc_key<N>(fx, fz);
         }
         fill += __popc(mask);
     };
@@ -995,21 +1648,9 @@ __global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_
         }
     };
     // the sources, 32 a step
-    if (GVDB2_SC_PREFETCH) {
-        // the next step's reads are in flight while this step's records are
-        // built and a full chunk is added
-        Src nxt = fetch(0);
-        for (uint32_t vb = 0; vb < total_src; vb += 32) {
-            const Src cur = nxt;
-            if (vb + 32 < total_src) nxt = fetch(vb + 32);
-            flush_if_full();
-            build(cur);
-        }
-    } else {
-        for (uint32_t vb = 0; vb < total_src; vb += 32) {
-            flush_if_full();
-            build(fetch(vb));
-        }
+    for (uint32_t vb = 0; vb < total_src; vb += 32) {
+        flush_if_full();
+        build(fetch(vb));
     }
     if (fill > 0) {
         sc_sort_chunk(C, fill, lane);
@@ -1026,26 +1667,69 @@ __global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_
                     acc[z][xp][c] = (c & 1) ? make_float2(a0.y, a1.y) : make_float2(a0.x, a1.x);
                 }
     }
-    // cells with a dense cell around get its partials from k_scatter_merge;
-    // one without sources of its own (all zero here) is listed as ~cell and
-    // left for the merge to write
-    if (any_part) {
-        if (lane == 0) S.merge_list[atomicAdd(S.merge_cnt, 1u)] = total_src == 0 ? ~(int32_t)cell : (int32_t)cell;
-        if (total_src == 0) return;
-    }
-    // each lane writes its 4 x 4 voxels of every channel once
-    const int a = S.apron, tl = S.tile;
-    const int64_t base = slot * S.tvox + (int64_t)(kCell * cx + 4 * q + a);
+    // the sums, channel by channel in z-major order, over the chunk; then out of
+    // it in whole rows
+    static_assert(sizeof(ScChunk) >= 512 * 4 * sizeof(float), "a cell's sums fit the chunk");
+    __syncwarp();
+    float *sums = reinterpret_cast<float *>(&C);
 #pragma unroll
     for (int zz = 0; zz < 4; zz++)
 #pragma unroll
-        for (int c = 0; c < NCH; c++) {
-            float *dst = S.chan[c] + base + ((int64_t)(kCell * cz + 4 * h + zz + a) * tl + (kCell * cy + y + a)) * tl;
-            dst[0] = acc[zz][0][c].x;
-            dst[1] = acc[zz][0][c].y;
-            dst[2] = acc[zz][1][c].x;
-            dst[3] = acc[zz][1][c].y;
-        }
+        for (int c = 0; c < NCH; c++)
+            *reinterpret_cast<float4 *>(sums + c * 512 + (4 * h + zz) * 64 + y * 8 + 4 * q) =
+                make_float4(acc[zz][0][c].x, acc[zz][0][c].y, acc[zz][1][c].x, acc[zz][1][c].y);
+    __syncwarp();
+    const int a = S.apron, tl = S.tile;
+    const int64_t base = slot * S.tvox + ((int64_t)(kCell * cz + a) * tl + (kCell * cy + a)) * tl + (kCell * cx + a);
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        const int i = k * 32 + lane, row = i >> 3;
+        const int64_t at = base + ((int64_t)(row >> 3) * tl + (row & 7)) * tl + (i & 7);
+#pragma unroll
+        for (int c = 0; c < NCH; c++) S.chan[c][at] = sums[c * 512 + i];
+    }
+}
+
+// kScWarps cells per CTA at a time, a warp per cell, of the cells of more than
+// kLightOwn points (SplatArgs::owner_list).  Their number is known on the device
+// only: each warp takes every (blocks * kScWarps)-th cell.
+template <int KERNEL, int NCH>
+__device__ __forceinline__ void scatter_listed_cells(const SplatArgs &S, ScChunk &C, int64_t block, int64_t blocks,
+                                                     int lane, int warp) {
+    const int64_t count = S.cell_cnt[kCntOwner];
+    for (int64_t i = block * kScWarps + warp; i < count; i += blocks * kScWarps) {
+        const int64_t cell = S.owner_list[i];
+        if (!in_range(S.lim, cell, S.ncell, 28)) continue;
+        scatter_cell<KERNEL, NCH>(S, C, cell, lane);
+        __syncwarp(); // the next cell reuses the chunk
+    }
+}
+template <int KERNEL, int NCH>
+__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_cells(SplatArgs S) {
+    extern __shared__ __align__(16) unsigned char sc_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    scatter_listed_cells<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], blockIdx.x, gridDim.x, lane, warp);
+}
+
+// Both in one launch, k_scatter_cells's cells in the first `heavy` blocks: in
+// volumes of few cells the longest of these (a warp each) would otherwise run
+// alone.  The same sums, so the host may choose by size.
+template <int KERNEL, int NCH>
+constexpr size_t owner_smem_bytes() {
+    return std::max(sizeof(ScChunk) * kScWarps, sizeof(LightWarp<NCH>) * kLightWarps);
+}
+template <int KERNEL, int NCH>
+__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_owner(SplatArgs S, unsigned heavy) {
+    static_assert(kScWarps == kLightWarps, "one block size");
+    extern __shared__ __align__(16) unsigned char sc_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x < heavy) {
+        scatter_listed_cells<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], blockIdx.x, heavy, lane, warp);
+        return;
+    }
+    const int64_t cell = (int64_t)(blockIdx.x - heavy) * kLightWarps + warp;
+    if (cell < S.ncell)
+        scatter_light_cell<KERNEL, NCH>(S, reinterpret_cast<LightWarp<NCH> *>(sc_smem)[warp], cell, lane);
 }
 
 // Adds the dense cells' partials to the cells listed by k_scatter_cells
@@ -1087,17 +1771,23 @@ __global__ void __launch_bounds__(512) k_scatter_merge(SplatArgs S) {
         const int v = threadIdx.x;
         const uint4 row = *reinterpret_cast<const uint4 *>(kMergeMap<KERNEL>.src[v]);
         const uint32_t wr[4] = {row.x, row.y, row.z, row.w};
-        float add[NCH];
-#pragma unroll
-        for (int c = 0; c < NCH; c++) add[c] = 0.0f;
+        // all of a thread's reads are issued before the first add (a voxel far
+        // from every face has one source, one near a corner eight)
+        float val[8][NCH];
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             const uint32_t ent = (wr[m >> 1] >> (16 * (m & 1))) & 0xFFFFu;
             const int32_t e = ent != 0xFFFFu ? ne[ent >> 11] : -1;
-            if (e < 0) continue;
-            const float *src = S.part + (int64_t)e * NCH * X::E3 + (ent & 2047u);
+            const float *src = S.part + (int64_t)max(e, 0) * NCH * X::E3 + (ent & 2047u);
 #pragma unroll
-            for (int c = 0; c < NCH; c++) add[c] += __ldcs(src + c * X::E3);
+            for (int c = 0; c < NCH; c++) val[m][c] = e >= 0 ? __ldcs(src + c * X::E3) : 0.0f;
+        }
+        float add[NCH];
+#pragma unroll
+        for (int c = 0; c < NCH; c++) {
+            add[c] = val[0][c];
+#pragma unroll
+            for (int m = 1; m < 8; m++) add[c] += val[m][c];
         }
         const int vx = v & 7, vy = (v >> 3) & 7, vz = v >> 6;
         const int a = S.apron, tl = S.tile;
@@ -1177,9 +1867,9 @@ __device__ __forceinline__ void gather_point(const GatherArgs &G, int32_t pidx, 
     float wx[N], wy[N], wz[N], dx[N], dy[N], dz[N];
     int fx, fy, fz;
     if (MODE == kFwd) {
-        fx = T::eval(p.x, wx) + o.x - ox;
-        fy = T::eval(p.y, wy) + o.y - oy;
-        fz = T::eval(p.z, wz) + o.z - oz;
+        fx = T::eval_fine(p.x, wx) + o.x - ox;
+        fy = T::eval_fine(p.y, wy) + o.y - oy;
+        fz = T::eval_fine(p.z, wz) + o.z - oz;
     } else {
         fx = T::eval_d(p.x, wx, dx) + o.x - ox;
         fy = T::eval_d(p.y, wy, dy) + o.y - oy;
@@ -1262,28 +1952,6 @@ __device__ __forceinline__ void gather_point(const GatherArgs &G, int32_t pidx, 
 
 constexpr int kGatherThreads = 256; // threads of a k_gather_tile CTA
 constexpr int kGatherChunk = 1024;  // points ordered per pass
-
-// A voxel's channels side by side in the staged tile: one shared-memory
-// load per tap serves every channel.
-template <int NCH> struct GVec { using T = float4; };
-template <> struct GVec<1> { using T = float; };
-template <> struct GVec<2> { using T = float2; };
-template <int NCH>
-__device__ __forceinline__ void gvec_put(typename GVec<NCH>::T &v, const float (&g)[NCH]) {
-    if constexpr (NCH == 1) v = g[0];
-    else if constexpr (NCH == 2) v = make_float2(g[0], g[1]);
-    else if constexpr (NCH == 3) v = make_float4(g[0], g[1], g[2], 0.0f);
-    else v = make_float4(g[0], g[1], g[2], g[3]);
-}
-template <int NCH>
-__device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *g) {
-    if constexpr (NCH == 1) g[0] = v;
-    else if constexpr (NCH == 2) g[0] = v.x, g[1] = v.y;
-    else {
-        g[0] = v.x, g[1] = v.y, g[2] = v.z;
-        if constexpr (NCH == 4) g[3] = v.w;
-    }
-}
 
 template <int KERNEL, int NCH>
 constexpr size_t gather_tile_smem() {
@@ -1585,6 +2253,11 @@ gvdb2_status ensure_zeroed(Volume *v, DevBuf &b, size_t bytes) {
     return GVDB2_OK;
 }
 
+// Up to this many cells the owner-computes pass is one launch (k_scatter_owner):
+// above it the light cells, most of such a volume, gain more from the
+// occupancy of a kernel of their own.
+constexpr int64_t kOneLaunchCells = 1 << 16;
+
 // Scatter of up to 4 channels (one group): the channel amounts in bin order,
 // the dense cells' partial sums (a CTA per slice), then the owner-computes
 // pass over every cell of the active bricks (cells no stencil reaches get
@@ -1594,7 +2267,6 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     using X = ExtTile<KERNEL>;
     constexpr size_t smem = sizeof(ScChunk) * kScWarps;
     auto k = k_scatter_cells<KERNEL, NCH>;
-    GV_TRY(launch_smem(v, k, smem, "scatter"));
     GV_CUDA(v, v->bin_amt.ensure(sizeof(float4) * (size_t)std::max<int64_t>(v->bin_key.n, 1), v->stream));
     GV_CUDA(v, v->part_buf.ensure(sizeof(float) * (size_t)std::max<int64_t>(v->dense_cap * NCH * X::E3, 1), v->stream));
     GV_TRY(ensure_zeroed(v, v->part_acc, sizeof(int32_t) * (size_t)std::max<int64_t>(v->multi_cap * 2 * NCH * X::E3, 1)));
@@ -1611,17 +2283,43 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     // the list's count sits in its last 16 bytes
     S.merge_cnt = reinterpret_cast<uint32_t *>(v->merge_list.as<char>() + v->merge_list.bytes - 16);
     S.merge_list = v->merge_list.as<int32_t>();
+    S.owner_list = v->cell_owner.as<int32_t>();
     GV_CUDA(v, cudaMemsetAsync(S.merge_cnt, 0, sizeof(uint32_t), v->stream));
     if (v->bin_key.n > 0)
         k_pack_amounts<NCH><<<grid_for(v->bin_key.n, 256, 1ll << 31), 256, 0, v->stream>>>(S);
+    if constexpr (KERNEL == GVDB2_KERNEL_CUBIC2) {
+        if (v->rows_cap > 0) {
+            auto kr = k_scatter_rows<NCH>;
+            GV_TRY(launch_smem(v, kr, sizeof(RowSmem<NCH>), "scatter"));
+            kr<<<(unsigned)v->rows_cap, 64, sizeof(RowSmem<NCH>), v->stream>>>(
+                S, v->rows_list.as<int32_t>(), v->prank.as<int32_t>(), v->row_off.as<uint16_t>());
+        }
+    }
     if (v->work_cap > 0) {
         constexpr size_t ps = part_smem_bytes<KERNEL, NCH>();
         auto kp = k_scatter_part<KERNEL, NCH>;
         GV_TRY(launch_smem(v, kp, ps, "scatter"));
         kp<<<(unsigned)v->work_cap, kPartThreads, ps, v->stream>>>(S);
     }
-    const int64_t blocks = (S.ncell + kScWarps - 1) / kScWarps;
-    if (blocks > 0) k<<<(unsigned)blocks, 32 * kScWarps, smem, v->stream>>>(S);
+    if (S.ncell > 0) {
+        // blocks for the cells of more than kLightOwn points: a warp each, but no more than 16 rounds
+        const int64_t heavy = std::min<int64_t>({S.ncell, v->bin_key.n / (kLightOwn + 1), (int64_t)64 * kSmCount * kScWarps});
+        const unsigned hb = (unsigned)((heavy + kScWarps - 1) / kScWarps);
+        const unsigned lb = (unsigned)((S.ncell + kLightWarps - 1) / kLightWarps);
+        if (S.ncell <= kOneLaunchCells) {
+            constexpr size_t os = owner_smem_bytes<KERNEL, NCH>();
+            auto ko = k_scatter_owner<KERNEL, NCH>;
+            GV_TRY(launch_smem(v, ko, os, "scatter"));
+            ko<<<hb + lb, 32 * kScWarps, os, v->stream>>>(S, hb);
+        } else {
+            constexpr size_t ls = sizeof(LightWarp<NCH>) * kLightWarps;
+            auto kl = k_scatter_light<KERNEL, NCH>;
+            GV_TRY(launch_smem(v, kl, ls, "scatter"));
+            GV_TRY(launch_smem(v, k, smem, "scatter"));
+            if (hb > 0) k<<<hb, 32 * kScWarps, smem, v->stream>>>(S);
+            kl<<<lb, 32 * kLightWarps, ls, v->stream>>>(S);
+        }
+    }
     // a cell with a dense cell among its 27 neighbours: at most 27 per dense cell
     const int64_t merge_grid = std::min<int64_t>(S.ncell, 27 * v->dense_cap);
     if (merge_grid > 0) k_scatter_merge<KERNEL, NCH><<<(unsigned)merge_grid, 512, 0, v->stream>>>(S);
@@ -1642,8 +2340,23 @@ SplatArgs channel_group(const SplatArgs &S, int first, int count) {
     return G;
 }
 
+// The dense cells' points in row order, once per binning.  prank, the ranks
+// that the binning is done with, holds the order.
+gvdb2_status sort_rows(Volume *v, const SplatArgs &S0) {
+    if (v->rows_sorted || v->rows_cap == 0) return GVDB2_OK;
+    GV_CUDA(v, v->row_off.ensure(sizeof(uint16_t) * kRowOff * (size_t)v->dense_cap, v->stream));
+    SplatArgs S = S0;
+    S.dense_cap = v->dense_cap;
+    k_sort_rows<<<(unsigned)v->rows_cap, kSortThreads, 0, v->stream>>>(S, v->rows_list.as<int32_t>(),
+                                                                       v->prank.as<int32_t>(), v->row_off.as<uint16_t>());
+    GV_CUDA(v, cudaGetLastError());
+    v->rows_sorted = true;
+    return GVDB2_OK;
+}
+
 template <int KERNEL>
 gvdb2_status scatter_groups(Volume *v, const SplatArgs &S) {
+    if (KERNEL == GVDB2_KERNEL_CUBIC2) GV_TRY(sort_rows(v, S));
     for (int first = 0; first < S.nch; first += 4) {
         const int cnt = std::min(4, S.nch - first);
         const SplatArgs G = channel_group(S, first, cnt);

@@ -3,7 +3,7 @@ their tiles, remainders, the smallest and the largest of their range."""
 import numpy as np
 import pytest
 
-from _helpers import make_oracle
+from _helpers import REL_TOL, interior, make_oracle, rel_err
 from test_gpu_topology import compare_topology, gpu_volume
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +40,29 @@ def test_parent_levels(gvdb2_mod, oracle_mod, lo, hi):
     v = gpu_volume(gvdb2_mod, pts)
     v.RebuildTopology(len(pts), 2.0)
     compare_topology(v, o)
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("nch", [1, 2, 3, 4])
+@pytest.mark.parametrize("per_cell", [1, 32, 33, 96, 97, 129, 193, 767, 768, 2048, 2049])
+def test_scatter_cell_classes(gvdb2_mod, oracle_mod, kernel, nch, per_cell):
+    """One cell of per_cell points among empty ones, at a cell corner of a 16^3 brick so that neighbours in and beyond
+    the brick get them: the ends of a 32-source step, of a source list, and of each class of cells (light, neighbour of
+    a heavy one, owner-computes, fixed point, rows); against the FP64 oracle within 1e-5 of the largest value."""
+    import torch
+    rng = np.random.default_rng(22)
+    pts = np.concatenate([rng.uniform(80.0, 87.999 if per_cell > 128 else 80.4, (per_cell, 3)), [[100.0, 100.0, 100.0]]]).astype(np.float32)
+    vel = rng.normal(size=(len(pts), 4)).astype(np.float32)
+    chans = list(range(nch))
+    cfg = (3, 3, 3, 3, 4)
+    o = make_oracle(oracle_mod, cfg, chans)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.update_atlas()
+    v = gpu_volume(gvdb2_mod, pts, cfg, chans)
+    v.RebuildTopology(len(pts), 2.0)
+    v.UpdateAtlas()
+    tv = torch.from_numpy(vel).cuda()
+    v.ScatterKernel(kernel, len(pts), chans, attrs=[(tv, c) for c in chans])
+    o.scatter_kernel(kernel, pts, chans, attrs=[vel[:, c] for c in chans])
+    for c in chans:
+        assert rel_err(interior(v.atlas(c), 1), interior(o.atlas(c), 1)) < REL_TOL
