@@ -1852,14 +1852,21 @@ __device__ __forceinline__ void gather_point_at(const GatherArgs &G, int32_t pid
     }
 }
 
-// One point of a gather, in any mode.  fetch(x, y, z, g) gives g[c], the
-// value of channel c at tap (x, y, z) of the cell's extended frame, whose
-// origin (ox, oy, oz) is the cell's first voxel minus H.
-template <int KERNEL, int MODE, int NCH, class Fetch>
+// One point of a gather, in any mode.  rows(fx, fy, fz) takes the point's first
+// taps in the cell's extended frame, whose origin (ox, oy, oz) is the cell's
+// first voxel minus H, and gives row(ty, tz, g), which reads the channels of
+// that row's taps into g[tx][c].
+//
+// The sums are taken axis by axis (x in a row, rows of a plane, planes), each
+// with one axis's weights and slopes: 5 products a tap and channel in all modes
+// together instead of up to 8, and no products of weights.  Where only the
+// position's gradient is wanted (kGatherBwd) the channels are summed first.
+template <int KERNEL, int MODE, int NCH, class Rows>
 __device__ __forceinline__ void gather_point(const GatherArgs &G, int32_t pidx, int64_t j, int ox, int oy, int oz,
-                                             const Fetch &fetch) {
+                                             const Rows &rows) {
     using T = Taps<KERNEL>;
     constexpr int N = T::N;
+    constexpr int NS = MODE == kGatherBwd ? 1 : NCH; // channels of the sums
     if (!in_range(G.lim, pidx, G.lim.nentry, 13)) return;
     float3 p;
     int3 o;
@@ -1883,33 +1890,53 @@ __device__ __forceinline__ void gather_point(const GatherArgs &G, int32_t pidx, 
 #pragma unroll
         for (int k = 0; k < N; k++) wx[k] = wy[k] = wz[k] = dx[k] = dy[k] = dz[k] = 0.0f;
     }
-    float sum[NCH], gx[NCH], gy[NCH], gz[NCH];
+    float go[NCH];
+    if (MODE == kGatherBwd)
 #pragma unroll
-    for (int c = 0; c < NCH; c++) sum[c] = gx[c] = gy[c] = gz[c] = 0.0f;
+        for (int c = 0; c < NCH; c++) go[c] = G.grad_out[(int64_t)pidx * NCH + c];
+    const auto row = rows(fx, fy, fz);
+    float sum[NS], gx[NS], gy[NS], gz[NS];
+#pragma unroll
+    for (int c = 0; c < NS; c++) sum[c] = gx[c] = gy[c] = gz[c] = 0.0f;
 #pragma unroll
     for (int tz = 0; tz < N; tz++) {
+        float pl[NS], plx[NS], ply[NS]; // the plane's sums: value, slope along x, along y
+#pragma unroll
+        for (int c = 0; c < NS; c++) pl[c] = plx[c] = ply[c] = 0.0f;
 #pragma unroll
         for (int ty = 0; ty < N; ty++) {
-            const float wyz = wy[ty] * wz[tz];
-            float dyz = 0.0f, ydz = 0.0f;
-            if (MODE != kFwd) {
-                dyz = dy[ty] * wz[tz];
-                ydz = wy[ty] * dz[tz];
-            }
+            float gv[N][NCH];
+            row(ty, tz, gv);
+            if (MODE == kGatherBwd)
 #pragma unroll
-            for (int tx = 0; tx < N; tx++) {
-                float gv[NCH];
-                fetch(fx + tx, fy + ty, fz + tz, gv);
+                for (int tx = 0; tx < N; tx++) {
+                    float g = go[0] * gv[tx][0];
 #pragma unroll
-                for (int c = 0; c < NCH; c++) {
-                    const float g = gv[c];
-                    if (MODE != kGatherBwd) sum[c] = fmaf(g, wx[tx] * wyz, sum[c]);
-                    if (MODE != kFwd) {
-                        gx[c] = fmaf(g, dx[tx] * wyz, gx[c]);
-                        gy[c] = fmaf(g, wx[tx] * dyz, gy[c]);
-                        gz[c] = fmaf(g, wx[tx] * ydz, gz[c]);
-                    }
+                    for (int c = 1; c < NCH; c++) g = fmaf(go[c], gv[tx][c], g);
+                    gv[tx][0] = g;
                 }
+#pragma unroll
+            for (int c = 0; c < NS; c++) {
+                float r = gv[0][c] * wx[0], rx = 0.0f;
+#pragma unroll
+                for (int tx = 1; tx < N; tx++) r = fmaf(gv[tx][c], wx[tx], r);
+                pl[c] = fmaf(r, wy[ty], pl[c]);
+                if (MODE != kFwd) {
+                    rx = gv[0][c] * dx[0];
+#pragma unroll
+                    for (int tx = 1; tx < N; tx++) rx = fmaf(gv[tx][c], dx[tx], rx);
+                    plx[c] = fmaf(rx, wy[ty], plx[c]);
+                    ply[c] = fmaf(r, dy[ty], ply[c]);
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NS; c++) {
+            if (MODE != kGatherBwd) sum[c] = fmaf(pl[c], wz[tz], sum[c]);
+            if (MODE != kFwd) {
+                gx[c] = fmaf(plx[c], wz[tz], gx[c]);
+                gy[c] = fmaf(ply[c], wz[tz], gy[c]);
+                gz[c] = fmaf(pl[c], dz[tz], gz[c]);
             }
         }
     }
@@ -1936,17 +1963,9 @@ __device__ __forceinline__ void gather_point(const GatherArgs &G, int32_t pidx, 
             G.grad_pos[3 * (int64_t)pidx + 2] = gp2;
         }
     } else {
-        float gp0 = 0.0f, gp1 = 0.0f, gp2 = 0.0f;
-#pragma unroll
-        for (int c = 0; c < NCH; c++) {
-            const float go = G.grad_out[(int64_t)pidx * NCH + c];
-            gp0 += go * gx[c];
-            gp1 += go * gy[c];
-            gp2 += go * gz[c];
-        }
-        G.grad_pos[3 * (int64_t)pidx + 0] = gp0;
-        G.grad_pos[3 * (int64_t)pidx + 1] = gp1;
-        G.grad_pos[3 * (int64_t)pidx + 2] = gp2;
+        G.grad_pos[3 * (int64_t)pidx + 0] = gx[0];
+        G.grad_pos[3 * (int64_t)pidx + 1] = gy[0];
+        G.grad_pos[3 * (int64_t)pidx + 2] = gz[0];
     }
 }
 
@@ -2023,7 +2042,13 @@ __device__ __forceinline__ void gather_tile_cell(const GatherArgs &G, int64_t bl
     }
     const Node &nd = G.leaves[leaf];
     const int ox = nd.mPos[0] + kCell * cx - H, oy = nd.mPos[1] + kCell * cy - H, oz = nd.mPos[2] + kCell * cz - H;
-    auto fetch = [&](int x, int y, int z, float g[NCH]) { gvec_get<NCH>(tile[(z * ht + y) * ht + x], g); };
+    auto rows = [&](int fx, int fy, int fz) {
+        const V *first = tile + (fz * ht + fy) * ht + fx;
+        return [first](int ty, int tz, float (&g)[N][NCH]) {
+#pragma unroll
+            for (int tx = 0; tx < N; tx++) gvec_get<NCH>(first[(tz * ht + ty) * ht + tx], g[tx]);
+        };
+    };
     for (uint32_t cb = beg; cb < end; cb += kGatherChunk) {
         const int cnt = (int)min((uint32_t)kGatherChunk, end - cb);
         for (int i = threadIdx.x; i <= nkeys; i += kGatherThreads) hist[i] = 0;
@@ -2074,7 +2099,7 @@ __device__ __forceinline__ void gather_tile_cell(const GatherArgs &G, int64_t bl
         for (int j = threadIdx.x; j < cnt; j += kGatherThreads) order[hist[key[j]] + rank[j]] = (uint16_t)j;
         __syncthreads();
         for (int j = threadIdx.x; j < cnt; j += kGatherThreads)
-            gather_point<KERNEL, MODE, NCH>(G, G.perm[cb + order[j]], (int64_t)cb + order[j], ox, oy, oz, fetch);
+            gather_point<KERNEL, MODE, NCH>(G, G.perm[cb + order[j]], (int64_t)cb + order[j], ox, oy, oz, rows);
         __syncthreads(); // the order arrays are reused by the next chunk
     }
 }
@@ -2090,7 +2115,7 @@ constexpr int kLightPack = 4;
 
 template <int KERNEL, int MODE, int NCH>
 __device__ __forceinline__ void gather_light_point(const GatherArgs &G, int64_t cell, int64_t entry) {
-    constexpr int H = Taps<KERNEL>::N / 2;
+    constexpr int N = Taps<KERNEL>::N, H = N / 2;
     int64_t slot;
     int cx, cy, cz;
     cell_coords(cell, G.m, G.m3, slot, cx, cy, cz);
@@ -2099,20 +2124,47 @@ __device__ __forceinline__ void gather_light_point(const GatherArgs &G, int64_t 
     const Node &nd = G.leaves[leaf];
     const int fx0 = kCell * cx - H, fy0 = kCell * cy - H, fz0 = kCell * cz - H; // frame origin in the brick
     const int res = G.res0, a = G.apron, tl = G.tile;
-    auto fetch = [&](int x, int y, int z, float g[NCH]) {
-        const int lx = fx0 + x, ly = fy0 + y, lz = fz0 + z; // brick-local, may step into a neighbour
-        const int sx = lx < 0 ? -1 : (lx >= res ? 1 : 0), sy = ly < 0 ? -1 : (ly >= res ? 1 : 0),
-                  sz = lz < 0 ? -1 : (lz >= res ? 1 : 0);
-        const int d = (sz + 1) * 9 + (sy + 1) * 3 + (sx + 1);
-        int64_t ns = d == 13 ? slot : (int64_t)G.nbr27[slot * 27 + d];
-        if (ns >= 0 && !in_range(G.lim, ns, G.lim.nslot, 20)) ns = -1;
-        const int64_t off = ns * G.tvox + ((int64_t)(lz - sz * res + a) * tl + (ly - sy * res + a)) * tl +
-                            (lx - sx * res + a);
+    // Along each axis a stencil lies in one brick or in two, the first `cut` taps
+    // in the lower one; the two bricks' steps from this brick are s and s + 1 (or s
+    // again).  A tap's offset is the row's plus tx, in either brick's rows.
+    auto rows = [&](int fx, int fy, int fz) {
+        const int lx = fx0 + fx, ly = fy0 + fy, lz = fz0 + fz; // brick-local, may step into a neighbour
+        auto step = [&](int l) { return l < 0 ? -1 : (l >= res ? 1 : 0); };
+        const int sx = step(lx), sy = step(ly), sz = step(lz);
+        const int ex = step(lx + N - 1), ey = step(ly + N - 1), ez = step(lz + N - 1);
+        const int cutx = ex == sx ? N : (ex == 0 ? -lx : res - lx), cuty = ey == sy ? N : (ey == 0 ? -ly : res - ly),
+                  cutz = ez == sz ? N : (ez == 0 ? -lz : res - lz);
+        // element offset of the stencil's first tap in each of the up to 8 bricks;
+        // where there is none, one that stays below 0 for every tap
+        constexpr int64_t none = -(int64_t(1) << 40);
+        int64_t at[2][2][2];
 #pragma unroll
-        for (int c = 0; c < NCH; c++) g[c] = ns >= 0 ? __ldg(G.chan[c] + off) : 0.0f;
+        for (int k = 0; k < 8; k++) {
+            const int kx = k & 1 ? ex : sx, ky = k & 2 ? ey : sy, kz = k & 4 ? ez : sz;
+            const int d = (kz + 1) * 9 + (ky + 1) * 3 + (kx + 1);
+            // a brick that repeats another's steps is not read again
+            const bool same = ((k & 1) && ex == sx) || ((k & 2) && ey == sy) || ((k & 4) && ez == sz);
+            int64_t ns = same ? -1 : (d == 13 ? slot : (int64_t)G.nbr27[slot * 27 + d]);
+            if (ns >= 0 && !in_range(G.lim, ns, G.lim.nslot, 20)) ns = -1;
+            at[(k >> 2) & 1][(k >> 1) & 1][k & 1] =
+                ns < 0 ? none
+                       : ns * G.tvox + (((lz - kz * res + a) * tl + (ly - ky * res + a)) * tl + (lx - kx * res + a));
+        }
+        return [=, &G](int ty, int tz, float (&g)[N][NCH]) {
+            const bool by = ty >= cuty, bz = tz >= cutz;
+            const int r = (tz * tl + ty) * tl;
+            const int64_t o0 = (bz ? (by ? at[1][1][0] : at[1][0][0]) : (by ? at[0][1][0] : at[0][0][0])) + r;
+            const int64_t o1 = (bz ? (by ? at[1][1][1] : at[1][0][1]) : (by ? at[0][1][1] : at[0][0][1])) + r;
+#pragma unroll
+            for (int tx = 0; tx < N; tx++) {
+                const int64_t o = tx >= cutx ? o1 : o0;
+#pragma unroll
+                for (int c = 0; c < NCH; c++) g[tx][c] = o >= 0 ? __ldg(G.chan[c] + o + tx) : 0.0f;
+            }
+        };
     };
     gather_point<KERNEL, MODE, NCH>(G, G.perm[entry], entry, nd.mPos[0] + fx0, nd.mPos[1] + fy0, nd.mPos[2] + fz0,
-                                    fetch);
+                                    rows);
 }
 
 template <int KERNEL, int MODE, int NCH>
@@ -2164,11 +2216,16 @@ __device__ __forceinline__ void gather_light_cells(const GatherArgs &G, int64_t 
 // One fused launch measured slower: the light path's registers (66) halved
 // the tiles' occupancy.
 template <int KERNEL, int MODE, int NCH>
-__global__ void __launch_bounds__(kGatherThreads) k_gather_tile(GatherArgs G) {
+__global__ void __launch_bounds__(kGatherThreads, MODE == kScatterBwd && NCH >= 3 ? 3 : 0) k_gather_tile(GatherArgs G) {
     gather_tile_cell<KERNEL, MODE, NCH>(G, blockIdx.x);
 }
+// The register budgets are measured: batched clouds (one channel) forward and two
+// adjoints 0.75 + 1.05 + 1.20 ms with the taps' offsets computed one by one (4,200
+// instructions a point), 0.44 + 0.54 + 0.61 with them per stencil at 80 registers,
+// 0.55 + 0.60 + 0.60 at 128; a sparse scene (3, 3 and 4 channels) 1.00 + 1.65 + 1.98
+// -> 0.67 + 0.72 + 1.08 ms at 128, 0.82 + 1.03 + 1.63 at 80, where it spills.
 template <int KERNEL, int MODE, int NCH>
-__global__ void __launch_bounds__(256) k_gather_light(GatherArgs G) {
+__global__ void __launch_bounds__(256, NCH == 1 ? 3 : 2) k_gather_light(GatherArgs G) {
     gather_light_cells<KERNEL, MODE, NCH>(G, blockIdx.x);
 }
 
