@@ -94,3 +94,35 @@ def test_gather_at_brick_corner(gvdb2_mod, oracle_mod, kernel, nch, per_cell):
     assert rel_err(v.GatherKernel(kernel, n, chans).cpu().numpy(), o.gather_kernel(kernel, pts, chans)) < REL_TOL
     gp = v.GatherDensityBackward(kernel, n, chans, torch.from_numpy(go).cuda()).cpu().numpy()
     assert rel_err(gp, o.gather_kernel_backward(kernel, pts, chans, go)) < REL_TOL
+
+
+@pytest.mark.parametrize("nch,cfg,apron", [(1, (3, 3, 3, 3, 3), 1), (2, (3, 3, 3, 3, 4), 2), (3, (3, 3, 3, 3, 2), 1),
+                                           (5, (3, 3, 3, 3, 3), 2)])
+def test_apron_channels(gvdb2_mod, nch, cfg, apron):
+    """Every channel's apron in one call, in groups of 4 and a remainder, for bricks of 4^3 to 16^3: copies of the
+    owners' interior values and the boundary value, exactly, and interiors left alone."""
+    import torch
+    rng = np.random.default_rng(24)
+    pts = rng.uniform(70.0, 110.0, (200, 3)).astype(np.float32)
+    chans = list(range(nch))
+    v = gpu_volume(gvdb2_mod, pts, cfg, chans, apron)
+    v.RebuildTopology(len(pts), 2.0)
+    v.UpdateAtlas()
+    tiles = []
+    for c in chans:
+        t = rng.integers(0, 1 << 20, v.atlas(c).shape).astype(np.float32)
+        v.atlas_tensor(c).copy_(torch.from_numpy(t).cuda())
+        tiles.append(t)
+    v.UpdateApron(-1, -7.0)
+    pos = v.atlas_map()["mPos"][:len(tiles[0])]
+    where = {tuple(p): s for s, p in enumerate(pos.tolist())}
+    res, t = 1 << cfg[4], tiles[0].shape[1]
+    for c in chans:
+        got = v.atlas(c)
+        for s in range(0, len(pos), max(1, len(pos) // 40)):
+            for z, y, x in ((0, 0, 0), (0, t - 1, apron), (apron, apron, t - 1), (t - 1, apron, 0), (apron, 0, t - 1)):
+                w = np.array((x, y, z)) - apron + pos[s]
+                own = where.get(tuple((w // res * res).tolist()))
+                lx, ly, lz = w % res + apron
+                assert got[s, z, y, x] == (-7.0 if own is None else tiles[c][own, lz, ly, lx])
+            assert np.array_equal(interior(got, apron)[s], interior(tiles[c], apron)[s])
