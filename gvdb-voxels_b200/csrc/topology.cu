@@ -727,7 +727,10 @@ __device__ __forceinline__ void bg_set(uint32_t *bits, int64_t bit) {
 // (the host then takes the hash path).  With SMEM the CTA first marks a
 // shared copy of both bitmaps (grid-stride over the points) and then ORs
 // its non-zero words into the global ones: a small grid would otherwise
-// put every point's atomics on the same few L2 lines.
+// put every point's atomics on the same few L2 lines.  Bound by instruction
+// issue (each point's box) over one read of the positions: 16.7M points 318 us
+// with a bounds check, an index and a bit for each of a box's bricks, 223 with a
+// run of bits along z at a time.
 template <bool SMEM>
 __global__ void k_mark_bits(PointsView pos, int64_t n, float3 orig, float radius, float kmax, int do_box, KeyGeom g,
                             BitGrid G, int32_t *status) {
@@ -757,47 +760,52 @@ __global__ void k_mark_bits(PointsView pos, int64_t n, float3 orig, float radius
             oo[1] = o.y;
             oo[2] = o.z;
         }
-        int64_t bit = -1;
-        int bx = 0, by = 0, bz = 0;
+        int bit = -1; // the grid holds at most 2^30 bits
         if (valid) {
-            bx = ((int)w[0] + oo[0]) >> g.log2r0;
-            by = ((int)w[1] + oo[1]) >> g.log2r0;
-            bz = ((int)w[2] + oo[2]) >> g.log2r0;
+            const int bx = ((int)w[0] + oo[0]) >> g.log2r0, by = ((int)w[1] + oo[1]) >> g.log2r0,
+                      bz = ((int)w[2] + oo[2]) >> g.log2r0;
             if (brick_in_root(g, bx, by, bz)) {
-                if (bg_in(G, bx, by, bz)) bit = bg_bit(G, bx, by, bz);
+                if (bg_in(G, bx, by, bz)) bit = (int)bg_bit(G, bx, by, bz);
                 else atomicOr(status, kDevCapacity);
             }
         }
-        // one atomic per distinct bit per warp
-        const unsigned peers = __match_any_sync(0xffffffffu, (unsigned long long)bit);
-        if (bit >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) {
-            if (SMEM) atomicOr(base + (bit >> 5), 1u << (bit & 31));
-            else bg_set(base, bit);
+        if (SMEM) {
+            if (bit >= 0 && !(base[bit >> 5] >> (bit & 31) & 1)) atomicOr(base + (bit >> 5), 1u << (bit & 31));
+        } else { // one atomic per distinct bit per warp
+            const unsigned peers = __match_any_sync(0xffffffffu, bit);
+            if (bit >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) bg_set(base, bit);
         }
         if (!valid || !do_box) continue;
         int lo[3], hi[3];
+        bool out = false;
+#pragma unroll
         for (int a = 0; a < 3; a++) {
             const int iw = (int)w[a];
             const int bmin = (int)((float)iw - radius);
             const int bmax = (int)((float)iw + kmax * radius);
             lo[a] = max(((bmin < 0 ? 0 : bmin) + oo[a]) >> g.log2r0, g.lo[a]); // clamped in the cloud's own space
             hi[a] = min((bmax + oo[a]) >> g.log2r0, g.lo[a] + g.span - 1);
+            out = out || lo[a] < G.o[a] || hi[a] >= G.o[a] + G.d[a];
         }
-        for (int x = lo[0]; x <= hi[0]; x++)
-            for (int y = lo[1]; y <= hi[1]; y++)
-                for (int z = lo[2]; z <= hi[2]; z++) {
-                    if (!bg_in(G, x, y, z)) {
-                        atomicOr(status, kDevCapacity);
-                        continue;
-                    }
-                    const int64_t bb = bg_bit(G, x, y, z);
+        if (out && lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2]) atomicOr(status, kDevCapacity);
+        lo[2] = max(lo[2], G.o[2]);
+        hi[2] = min(hi[2], G.o[2] + G.d[2] - 1);
+        // bits of one (x, y) are consecutive along z: a word's share of the run at
+        // once (the grid holds at most 2^30 bits)
+        for (int x = max(lo[0], G.o[0]); x <= min(hi[0], G.o[0] + G.d[0] - 1); x++)
+            for (int y = max(lo[1], G.o[1]); y <= min(hi[1], G.o[1] + G.d[1] - 1); y++) {
+                const int row = ((x - G.o[0]) * G.d[1] + (y - G.o[1])) * G.d[2] - G.o[2];
+                for (int b = row + lo[2]; b <= row + hi[2]; b = (b | 31) + 1) {
+                    const int last = min(row + hi[2], b | 31);
+                    const uint32_t m = (0xFFFFFFFFu >> (31 - (last - b))) << (b & 31);
+                    uint32_t *wd = box + (b >> 5);
                     if (SMEM) {
-                        const uint32_t m = 1u << (bb & 31);
-                        if (!(box[bb >> 5] & m)) atomicOr(box + (bb >> 5), m);
-                    } else {
-                        bg_set(box, bb);
+                        if (~*wd & m) atomicOr(wd, m);
+                    } else if (~__ldcg(wd) & m) {
+                        atomicOr(wd, m);
                     }
                 }
+            }
     }
     if (SMEM) {
         __syncthreads();
