@@ -251,7 +251,11 @@ __device__ __forceinline__ uint16_t quantize16(float x, float lo, float range) {
 // tests the sign after adding trans, the insert pass before, the fp16 insert
 // pass tests NOHIT and the sign on the translated position, all as in the
 // reference; an insert never writes past the counted capacity of its
-// subcell.
+// subcell.  Bound by an atomic add a visit and, in the inserts, by the 12-byte
+// entries they place.  The box's leaves are looked up once a brick, at most two
+// an axis, and not once a subcell: 4.2M points, 47.8M visits, 461 + 685 -> 321 +
+// 581 us to count and insert.  (Brick by brick, the lanes' loops diverge: 361 +
+// 683.  One add for the lanes of a warp that visit a subcell together: 508 + 938.)
 template <int PASS>
 __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const uint32_t *off, float *pnt,
                            int32_t *status) {
@@ -281,46 +285,87 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const u
     int mn[3], mx[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        mn[a] = ((int)(w[a] - A.radius) / A.sc) * A.sc;
+        mn[a] = max(((int)(w[a] - A.radius) / A.sc) * A.sc, 0);
         mx[a] = ((int)(w[a] + 1 + A.radius) / A.sc) * A.sc;
+        if (mx[a] < 0) return;
     }
-    for (int sx = mn[0]; sx <= mx[0]; sx += A.sc)
-        for (int sy = mn[1]; sy <= mx[1]; sy += A.sc)
-            for (int sz = mn[2]; sz <= mx[2]; sz += A.sc) {
-                if (sx < 0 || sy < 0 || sz < 0) continue;
-                int32_t leaf = leaf_at_brick(A.L, sx >> A.L.g.log2r0, sy >> A.L.g.log2r0, sz >> A.L.g.log2r0);
-                if (leaf < 0 || leaf >= A.nleaves) continue;
-                const Node &nd = A.leaves[leaf];
-                int lx = (sx - nd.mPos[0]) / A.sc, ly = (sy - nd.mPos[1]) / A.sc, lz = (sz - nd.mPos[2]) / A.sc;
-                int64_t idx = (int64_t)A.mapping[leaf] * A.scpb + ((int64_t)lz * A.scdim + ly) * A.scdim + lx;
-                if (idx < 0 || idx >= A.num_sc) continue;
-                if (PASS == 0) {
-                    atomicAdd(&cnt[idx], 1u);
-                } else {
-                    uint32_t o = atomicAdd(&cnt[idx], 1u);
-                    if (o >= cap[idx]) {
-                        atomicSub(&cnt[idx], 1u); // the list keeps its counted length
-                        atomicOr(status, kDevCapacity);
-                        continue;
-                    }
-                    int64_t at = (int64_t)off[idx] + o;
-                    if (PASS == 2) {
-                        A.q[3 * at + 0] = quantize16(w[0], A.pmin.x, A.prange.x);
-                        A.q[3 * at + 1] = quantize16(w[1], A.pmin.y, A.prange.y);
-                        A.q[3 * at + 2] = quantize16(w[2], A.pmin.z, A.prange.z);
-                        if (A.qvel) {
-                            const float3 u = load_f3(A.vel, i);
-                            A.qvel[3 * at + 0] = quantize16(u.x, A.vmin.x, A.vrange.x);
-                            A.qvel[3 * at + 1] = quantize16(u.y, A.vmin.y, A.vrange.y);
-                            A.qvel[3 * at + 2] = quantize16(u.z, A.vmin.z, A.vrange.z);
-                        }
-                    } else {
-                        pnt[3 * at + 0] = w[0];
-                        pnt[3 * at + 1] = w[1];
-                        pnt[3 * at + 2] = w[2];
-                    }
-                }
+    const int lr = A.L.g.log2r0, rm = (1 << lr) - 1, ls = __ffs(A.sc) - 1; // a power of two, as it divides the brick
+    // first subcell of a brick's subcells, or -1
+    auto first_of = [&](int bx, int by, int bz) {
+        const int32_t leaf = leaf_at_brick(A.L, bx, by, bz);
+        return leaf < 0 || leaf >= A.nleaves ? int64_t(-1) : (int64_t)A.mapping[leaf] * A.scpb;
+    };
+    auto place = [&](int64_t idx, uint32_t o) {
+        if (o >= cap[idx]) {
+            atomicSub(&cnt[idx], 1u); // the list keeps its counted length
+            atomicOr(status, kDevCapacity);
+            return;
+        }
+        const int64_t at = (int64_t)off[idx] + o;
+        if (PASS == 2) {
+            A.q[3 * at + 0] = quantize16(w[0], A.pmin.x, A.prange.x);
+            A.q[3 * at + 1] = quantize16(w[1], A.pmin.y, A.prange.y);
+            A.q[3 * at + 2] = quantize16(w[2], A.pmin.z, A.prange.z);
+            if (A.qvel) {
+                const float3 u = load_f3(A.vel, i);
+                A.qvel[3 * at + 0] = quantize16(u.x, A.vmin.x, A.vrange.x);
+                A.qvel[3 * at + 1] = quantize16(u.y, A.vmin.y, A.vrange.y);
+                A.qvel[3 * at + 2] = quantize16(u.z, A.vmin.z, A.vrange.z);
             }
+        } else {
+            pnt[3 * at + 0] = w[0];
+            pnt[3 * at + 1] = w[1];
+            pnt[3 * at + 2] = w[2];
+        }
+    };
+    const int bx = mn[0] >> lr, by = mn[1] >> lr, bz = mn[2] >> lr;
+    const int ex = (mx[0] >> lr) - bx, ey = (mx[1] >> lr) - by, ez = (mx[2] >> lr) - bz;
+    if (ex > 1 || ey > 1 || ez > 1) { // a box over three bricks and more
+        for (int sx = mn[0]; sx <= mx[0]; sx += A.sc)
+            for (int sy = mn[1]; sy <= mx[1]; sy += A.sc)
+                for (int sz = mn[2]; sz <= mx[2]; sz += A.sc) {
+                    const int64_t f = first_of(sx >> lr, sy >> lr, sz >> lr);
+                    const int64_t idx = f + ((((sz & rm) >> ls) * A.scdim + ((sy & rm) >> ls)) * A.scdim + ((sx & rm) >> ls));
+                    if (f < 0 || idx >= A.num_sc) continue;
+                    const uint32_t o = atomicAdd(&cnt[idx], 1u);
+                    if (PASS != 0) place(idx, o);
+                }
+        return;
+    }
+    // the box's bricks, two an axis at most, each looked up once
+    int64_t f[2][2][2];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int kx = k & 1, ky = (k >> 1) & 1, kz = k >> 2;
+        f[kx][ky][kz] = kx <= ex && ky <= ey && kz <= ez ? first_of(bx + kx, by + ky, bz + kz) : int64_t(-1);
+    }
+    for (int sx = mn[0]; sx <= mx[0]; sx += A.sc) {
+        const bool x1 = (sx >> lr) != bx;
+        const int64_t g00 = x1 ? f[1][0][0] : f[0][0][0], g10 = x1 ? f[1][1][0] : f[0][1][0],
+                      g01 = x1 ? f[1][0][1] : f[0][0][1], g11 = x1 ? f[1][1][1] : f[0][1][1];
+        for (int sy = mn[1]; sy <= mx[1]; sy += A.sc) {
+            const bool y1 = (sy >> lr) != by;
+            const int64_t h0 = y1 ? g10 : g00, h1 = y1 ? g11 : g01;
+            const int row = ((sy & rm) >> ls) * A.scdim + ((sx & rm) >> ls);
+            // three along z at a time, their adds before the first entry is placed
+            for (int sz0 = mn[2]; sz0 <= mx[2]; sz0 += 3 * A.sc) {
+                int64_t idx[3];
+                uint32_t o[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    const int sz = sz0 + k * A.sc;
+                    const int64_t h = (sz >> lr) != bz ? h1 : h0;
+                    idx[k] = h + ((sz & rm) >> ls) * (A.scdim * A.scdim) + row;
+                    if (sz > mx[2] || h < 0 || idx[k] >= A.num_sc) idx[k] = -1;
+                    if (idx[k] >= 0) o[k] = atomicAdd(&cnt[idx[k]], 1u);
+                }
+                if (PASS != 0)
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        if (idx[k] >= 0) place(idx[k], o[k]);
+            }
+        }
+    }
 }
 
 // gvdbCalcSubcellPos (P:677-694), a thread per subcell of every pool leaf

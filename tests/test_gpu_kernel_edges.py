@@ -9,18 +9,20 @@ from test_gpu_topology import compare_topology, gpu_volume
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("radius", [0.4, 2.0, 9.5])
 @pytest.mark.parametrize("sc,cfg", [(2, (3, 3, 3, 3, 3)), (8, (3, 3, 3, 3, 3)), (4, (3, 3, 3, 3, 5)), (16, (3, 3, 3, 3, 5))])
-def test_subcell_table(gvdb2_mod, oracle_mod, sc, cfg):
-    """Every subcell's node and corner, for 1, 8, 64 and 512 subcells a brick, against the oracle (exact)."""
+def test_subcell_table(gvdb2_mod, oracle_mod, sc, cfg, radius):
+    """Every subcell's node, corner and list length, for 1, 8, 64 and 512 subcells a brick and boxes over one brick to
+    four, against the oracle (exact)."""
     rng = np.random.default_rng(20)
     pts = rng.uniform(70.0, 170.0, (3001, 3)).astype(np.float32)
     o = make_oracle(oracle_mod, cfg)
     assert o.rebuild_topology(pts, 2.0) == 0
-    o.insert_points_subcell(sc, pts, 2.0)
+    ln = o.insert_points_subcell(sc, pts, radius)
     cnt, nid, pos = o.subcells()
     v = gpu_volume(gvdb2_mod, pts, cfg)
     v.RebuildTopology(len(pts), 2.0)
-    v.InsertPointsSubcell(sc, len(pts), 2.0)
+    assert v.InsertPointsSubcell(sc, len(pts), radius) == ln
     g = v.subcells(len(cnt))
     for a, b in zip(g, (cnt, nid, pos)):
         assert np.array_equal(a, b)
@@ -31,14 +33,16 @@ def test_subcell_table(gvdb2_mod, oracle_mod, sc, cfg):
     ((68.0, 70.0, 66.0), (69.0, 71.0, 320.0)),      # one brick thick, several parents long
     ((61.0, 3.0, 509.0), (67.0, 260.0, 900.0)),     # parents that start inside the grid, two levels of them
 ])
-def test_parent_levels(gvdb2_mod, oracle_mod, lo, hi):
-    """Node pools and child lists of small and thin brick grids, against the oracle (exact)."""
+@pytest.mark.parametrize("radius", [2.0, 45.0])
+def test_parent_levels(gvdb2_mod, oracle_mod, lo, hi, radius):
+    """Node pools and child lists of small and thin brick grids, with activation boxes of one brick and of 18 (runs over
+    word ends, boxes cut at the root), against the oracle (exact)."""
     rng = np.random.default_rng(21)
     pts = rng.uniform(lo, hi, (400, 3)).astype(np.float32)
     o = make_oracle(oracle_mod)
-    assert o.rebuild_topology(pts, 2.0) == 0
+    assert o.rebuild_topology(pts, radius) == 0
     v = gpu_volume(gvdb2_mod, pts)
-    v.RebuildTopology(len(pts), 2.0)
+    v.RebuildTopology(len(pts), radius)
     compare_topology(v, o)
 
 
@@ -126,3 +130,27 @@ def test_apron_channels(gvdb2_mod, nch, cfg, apron):
                 lx, ly, lz = w % res + apron
                 assert got[s, z, y, x] == (-7.0 if own is None else tiles[c][own, lz, ly, lx])
             assert np.array_equal(interior(got, apron)[s], interior(tiles[c], apron)[s])
+
+
+@pytest.mark.parametrize("levelset", [False, True])
+@pytest.mark.parametrize("per_list", [1, 2, 63, 64, 65, 129])
+def test_voxel_gathers_list_ends(gvdb2_mod, oracle_mod, levelset, per_list):
+    """4^3 subcells with lists of one point, of odd and even lengths and around the 64 points staged at a time; against
+    the FP64 oracle within 1e-5 of the largest value."""
+    rng = np.random.default_rng(25)
+    pts = np.concatenate([rng.uniform(82.0, 82.9, (per_list, 3)), [[100.0, 100.0, 100.0]]]).astype(np.float32)
+    o = make_oracle(oracle_mod)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.update_atlas()
+    v = gpu_volume(gvdb2_mod, pts)
+    v.RebuildTopology(len(pts), 2.0)
+    v.UpdateAtlas()
+    ln = v.InsertPointsSubcell(4, len(pts), 0.5)
+    assert o.insert_points_subcell(4, pts, 0.5) == ln
+    if levelset:
+        v.GatherLevelSet(4, len(pts), 1.5, (0, 0, 0), ln, 0)
+        o.gather_level_set(4, 1.5, 0)
+    else:
+        v.GatherDensity(4, len(pts), 1.5, (0, 0, 0), ln, 0)
+        o.gather_density(4, 1.5, 0)
+    assert rel_err(interior(v.atlas(0), 1), interior(o.atlas(0), 1)) < REL_TOL
