@@ -94,7 +94,7 @@ gvdb2_status gvdb2_create(gvdb2_volume **out, int device) {
     gvdb2_volume *h = new (std::nothrow) gvdb2_volume();
     if (!h) return GVDB2_ERR_NOMEM;
     h->v.device = device;
-    if (cudaMallocHost(&h->v.host_small, 128) != cudaSuccess) {
+    if (cudaMallocHost(&h->v.host_small, gvdb2::kHostSmallBytes) != cudaSuccess) {
         delete h;
         return GVDB2_ERR_NOMEM;
     }
@@ -492,9 +492,10 @@ gvdb2_status gvdb2_get_info(gvdb2_volume *h, gvdb2_info *out) {
     CHECK_HANDLE(h);
     if (!out) return GVDB2_ERR_ARG;
     Volume *v = VOL(h);
+    int64_t cells = -1;
+    GV_TRY(gvdb2::flush_status(v, &cells));
     cudaError_t e = cudaStreamSynchronize(v->stream);
     if (e != cudaSuccess) return gvdb2::cuda_fail(v, e, "get_info");
-    GV_TRY(gvdb2::flush_status(v));
     std::memset(out, 0, sizeof(*out));
     out->depth = v->depth;
     out->top_level = v->top_level();
@@ -521,13 +522,7 @@ gvdb2_status gvdb2_get_info(gvdb2_volume *h, gvdb2_info *out) {
         out->vox_res[a] = v->vox_res[a];
         out->vox_res_max[a] = v->vox_res_max[a];
     }
-    out->splat_cells = -1;
-    if (v->bin_key.valid && v->cell_cnt.p) {
-        uint32_t c3[3] = {0, 0, 0};
-        e = cudaMemcpy(c3, v->cell_cnt.p, sizeof(c3), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return gvdb2::cuda_fail(v, e, "get_info");
-        out->splat_cells = (int64_t)c3[0] + c3[1] + c3[2];
-    }
+    out->splat_cells = cells;
     return GVDB2_OK;
 }
 

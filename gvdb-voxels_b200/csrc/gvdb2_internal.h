@@ -90,6 +90,8 @@ struct DevBuf {
     template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+constexpr size_t kHostSmallBytes = 192; // pinned mirror of the small device words and the cell counts
+
 struct Volume {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -167,7 +169,9 @@ struct Volume {
     int64_t lev_count[kMaxLev][2] = {{0}};
     DevBuf tmp_a, tmp_b, tmp_c, scratch;
     DevBuf dev_small;         // small device words: counters, status, bbox
-    void *host_small = nullptr; // pinned mirror of dev_small
+    void *host_small = nullptr; // pinned mirror of dev_small, then of cell_cnt
+    DevBuf scan_sums;         // tile sums of exclusive_scan_u32
+    bool cells_read = false;  // the mirror of cell_cnt is the current bins'
 
     // batched clouds (gvdb2_batch_points): the packed positions
     DevBuf batch_pos, batch_cloud, batch_origin;
@@ -324,8 +328,9 @@ gvdb2_status clear_channel(Volume *v, int chan);
 gvdb2_status compute_bounds(Volume *v);
 gvdb2_status sync_counts(Volume *v);
 // reads back the small device words when a full rebuild's status check is
-// pending and reports its error, if any
-gvdb2_status flush_status(Volume *v);
+// pending and reports its error, if any; with `cells`, the number of cells that
+// hold points (left alone when there are no bins)
+gvdb2_status flush_status(Volume *v, int64_t *cells = nullptr);
 // the small device word the splat kernels flag an out-of-range index in
 // (nullptr before the first rebuild)
 int32_t *splat_guard_word(Volume *v);

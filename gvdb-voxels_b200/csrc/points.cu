@@ -69,8 +69,9 @@ __device__ __forceinline__ int region_axis(float w, int cell_lo) {
 
 template <int KERNEL>
 __global__ void k_bin_count(PointsView pos, int64_t n, float3 trans, LeafLookup L, const int32_t *leaf_slot, int m,
-                            uint32_t *cnt, int32_t *pbin, int32_t *prank) {
+                            uint32_t *cnt, int32_t *pbin, int32_t *prank, uint32_t *cell_cnt) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kCntWords) cell_cnt[i] = 0; // for k_cell_list
     int32_t bin = -1;
     if (i < n) {
         float3 p = load_f3(pos, i);
@@ -99,12 +100,6 @@ __global__ void k_bin_count(PointsView pos, int64_t n, float3 trans, LeafLookup 
     } else if (i < n) {
         pbin[i] = -1;
     }
-}
-
-// bin_off[c] = reg_off[c * 27]: each cell's first point (c = ncell: the end)
-__global__ void k_cell_off(const uint32_t *reg_off, int64_t ncell, uint32_t *bin_off) {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c <= ncell) bin_off[c] = reg_off[c * kRegions];
 }
 
 // keys for the stable (deterministic) binning: bin id, unbinned last
@@ -159,12 +154,16 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // neighbour of more than kHeavyFace (not dense either) are listed in `owner`.  It depends on
 // the cell and its neighbours alone, so that a cloud of a batch gets what a
 // volume of its own gets.
-__global__ void k_cell_list(const uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int32_t *part,
+// reg_off holds each (cell, region) bin's first entry; off[c] = reg_off[27 c], each
+// cell's (c = ncell: the end), is written for the kernels that follow.
+__global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int32_t *part,
                             int32_t *owner, int32_t *rows, int4 *work, uint32_t *cnt, const int32_t *nbr27, int m,
                             uint32_t dense_min,
                             uint32_t slice, uint32_t light_max, bool cubic, bool rows_on) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t k = c < ncell ? off[c + 1] - off[c] : 0u;
+    const uint32_t first = c <= ncell ? reg_off[c * kRegions] : 0u;
+    if (c <= ncell) off[c] = first;
+    const uint32_t k = c < ncell ? reg_off[(c + 1) * kRegions] - first : 0u;
     const int cls = k == 0 ? -1 : (k > kHeavyCell ? kCntHuge : (k > light_max ? kCntHeavy : kCntLight));
     const unsigned act = __ballot_sync(0xffffffffu, cls >= 0);
     if (cls >= 0) {
@@ -195,7 +194,7 @@ __global__ void k_cell_list(const uint32_t *off, int64_t ncell, int32_t *list, i
             }
             if (ns < 0) continue;
             const int64_t n = ns * m * m * m + (nc[2] * m + nc[1]) * m + nc[0];
-            const uint32_t kn = off[n + 1] - off[n];
+            const uint32_t kn = reg_off[(n + 1) * kRegions] - reg_off[n * kRegions];
             own = kn > (uint32_t)kHeavyFace && !(dense_min > 0 && kn >= dense_min);
         }
     }
@@ -446,19 +445,18 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     GV_CUDA(v, v->reg_off.ensure(sizeof(uint32_t) * (size_t)(nreg + 1), s));
     GV_CUDA(v, v->bin_off.ensure(sizeof(uint32_t) * (size_t)(nbins + 1), s));
     GV_CUDA(v, cudaMemsetAsync(v->bin_cnt.p, 0, sizeof(uint32_t) * (size_t)(nreg + 1), s));
+    GV_CUDA(v, v->cell_cnt.ensure(sizeof(uint32_t) * kCntWords, s));
+    if (n == 0) GV_CUDA(v, cudaMemsetAsync(v->cell_cnt.p, 0, sizeof(uint32_t) * kCntWords, s));
     float3 t = make_float3(trans[0], trans[1], trans[2]);
     LeafLookup L = make_lookup(v);
     if (n > 0) {
         auto kc = kernel == GVDB2_KERNEL_TENT1 ? k_bin_count<GVDB2_KERNEL_TENT1> : k_bin_count<GVDB2_KERNEL_CUBIC2>;
         kc<<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(v->pos, n, t, L, v->leaf_slot.as<int32_t>(), m,
                                                      v->bin_cnt.as<uint32_t>(), v->pbin.as<int32_t>(),
-                                                     v->prank.as<int32_t>());
+                                                     v->prank.as<int32_t>(), v->cell_cnt.as<uint32_t>());
         GV_CUDA(v, cudaGetLastError());
     }
     GV_TRY(exclusive_scan_u32(v, v->bin_cnt.as<uint32_t>(), v->reg_off.as<uint32_t>(), nreg));
-    k_cell_off<<<grid_for(nbins + 1, 256, 1ll << 31), 256, 0, s>>>(v->reg_off.as<uint32_t>(), nbins,
-                                                                   v->bin_off.as<uint32_t>());
-    GV_CUDA(v, cudaGetLastError());
     if (n > 0 && v->deterministic) {
         // stable counting sort: a radix sort of (bin, point index) keeps each
         // bin's points in index order, independent of atomic timing; its key
@@ -500,13 +498,12 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     v->multi_cap = std::min<int64_t>(v->dense_cap, n / (sl + 1));
     GV_CUDA(v, v->rows_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(v->rows_cap, 1), s));
     GV_CUDA(v, v->part_work.ensure(sizeof(int4) * (size_t)std::max<int64_t>(v->work_cap, 1), s));
-    GV_CUDA(v, v->cell_cnt.ensure(sizeof(uint32_t) * kCntWords, s));
-    GV_CUDA(v, cudaMemsetAsync(v->cell_cnt.p, 0, sizeof(uint32_t) * kCntWords, s));
-
     v->cell_grid = v->heavy_grid = v->light_grid = 0;
+    v->cells_read = false;
+    if (nbins == 0) GV_CUDA(v, cudaMemsetAsync(v->bin_off.p, 0, sizeof(uint32_t), s));
     if (nbins > 0) {
-        const int g = grid_for(nbins, 256, 1ll << 31);
-        k_cell_list<<<g, 256, 0, s>>>(v->bin_off.as<uint32_t>(), nbins, v->cell_list.as<int32_t>(),
+        const int g = grid_for(nbins + 1, 256, 1ll << 31);
+        k_cell_list<<<g, 256, 0, s>>>(v->reg_off.as<uint32_t>(), v->bin_off.as<uint32_t>(), nbins, v->cell_list.as<int32_t>(),
                                       v->cell_light.as<int32_t>(), v->cell_part.as<int32_t>(), v->cell_owner.as<int32_t>(),
                                       v->rows_list.as<int32_t>(), v->part_work.as<int4>(), v->cell_cnt.as<uint32_t>(),
                                       v->nbr27.as<int32_t>(), m, (uint32_t)dmin, (uint32_t)v->tune_slice, (uint32_t)v->tune_light,

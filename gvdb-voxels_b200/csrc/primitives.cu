@@ -12,6 +12,7 @@ namespace {
 constexpr int kScanThreads = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int64_t kScanSums = 4096; // tiles whose sums each block adds up itself
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x) {
     const int lane = threadIdx.x & 31;
@@ -58,39 +59,51 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t *__
 }
 
 // Scan one tile: coalesced load into shared memory, per-thread serial scan
-// of kScanItems consecutive items, block scan of the thread sums.
+// of kScanItems consecutive items, block scan of the thread sums.  The sum of
+// the tiles before it is block_off[b] or, when that is null, added up from
+// `sums` (a few thousand at most) by every block: a launch of their own scan and
+// its memory cost more.  Padded by a word in 32, so that the threads' runs of 8
+// start in different banks.
+__device__ __forceinline__ int scan_at(int i) { return i + (i >> 5); }
 __global__ void __launch_bounds__(kScanThreads) k_scan_tile(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
-                                                            int64_t n, const uint32_t *__restrict__ block_off) {
-    __shared__ uint32_t tile[kScanTile];
+                                                            int64_t n, const uint32_t *__restrict__ block_off,
+                                                            const uint32_t *__restrict__ sums) {
+    __shared__ uint32_t tile[kScanTile + kScanTile / 32];
     __shared__ uint32_t sw[33];
     int64_t base = (int64_t)blockIdx.x * kScanTile;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
         int64_t i = base + (int64_t)j * kScanThreads + threadIdx.x;
-        tile[j * kScanThreads + threadIdx.x] = i < n ? in[i] : 0u;
+        tile[scan_at(j * kScanThreads + threadIdx.x)] = i < n ? in[i] : 0u;
     }
-    __syncthreads();
+    uint32_t off = block_off ? block_off[blockIdx.x] : 0u;
+    if (sums) {
+        uint32_t x = 0, excl;
+        for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanThreads) x += sums[b];
+        off = block_excl_scan(x, sw, excl);
+    } else {
+        __syncthreads();
+    }
     uint32_t v[kScanItems];
     uint32_t s = 0;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
-        v[j] = tile[threadIdx.x * kScanItems + j];
+        v[j] = tile[scan_at(threadIdx.x * kScanItems + j)];
         s += v[j];
     }
     uint32_t excl;
     uint32_t tot = block_excl_scan(s, sw, excl);
-    uint32_t off = block_off ? block_off[blockIdx.x] : 0u;
     uint32_t run = off + excl;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
-        tile[threadIdx.x * kScanItems + j] = run;
+        tile[scan_at(threadIdx.x * kScanItems + j)] = run;
         run += v[j];
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
         int64_t i = base + (int64_t)j * kScanThreads + threadIdx.x;
-        if (i < n) out[i] = tile[j * kScanThreads + threadIdx.x];
+        if (i < n) out[i] = tile[scan_at(j * kScanThreads + threadIdx.x)];
     }
     if (threadIdx.x == 0 && base + kScanTile >= n) out[n] = off + tot; // last tile writes the total
 }
@@ -175,7 +188,14 @@ gvdb2_status exclusive_scan_u32(Volume *v, const uint32_t *in, uint32_t *out, in
     }
     int64_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 1) {
-        k_scan_tile<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr);
+        k_scan_tile<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, nullptr);
+        GV_CUDA(v, cudaGetLastError());
+        return GVDB2_OK;
+    }
+    if (nb <= kScanSums) {
+        GV_CUDA(v, v->scan_sums.ensure(sizeof(uint32_t) * kScanSums, s));
+        k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, v->scan_sums.as<uint32_t>());
+        k_scan_tile<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, nullptr, v->scan_sums.as<uint32_t>());
         GV_CUDA(v, cudaGetLastError());
         return GVDB2_OK;
     }
@@ -185,7 +205,7 @@ gvdb2_status exclusive_scan_u32(Volume *v, const uint32_t *in, uint32_t *out, in
     k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums);
     gvdb2_status st = exclusive_scan_u32(v, sums, sums_scan, nb);
     if (st == GVDB2_OK) {
-        k_scan_tile<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums_scan);
+        k_scan_tile<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums_scan, nullptr);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(v, e, "k_scan_tile");
     }

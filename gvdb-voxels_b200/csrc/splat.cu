@@ -2240,12 +2240,27 @@ __global__ void __launch_bounds__(256, NCH == 1 ? 3 : 2) k_gather_light(GatherAr
     gather_light_cells<KERNEL, MODE, NCH>(G, blockIdx.x);
 }
 
-// Points outside every active brick: gathers and gradients are zero.
-__global__ void k_zero_unbinned(const int32_t *pbin, int64_t n, float *out, int64_t stride, int ncols) {
+// Points outside every active brick: gathers and gradients are zero.  Up to three
+// outputs of a call in one launch; when every point is binned (*binned == n, as
+// after a rebuild around the points) there is nothing to do.
+struct ZeroOuts {
+    float *out[3];
+    int64_t stride[3];
+    int cols[3];
+};
+__global__ void k_zero_unbinned(const int32_t *pbin, int64_t n, const uint32_t *binned, ZeroOuts Z) {
+    if ((int64_t)*binned == n) return;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !out) return;
+    if (i >= n) return;
     if (pbin[i] >= 0) return;
-    for (int c = 0; c < ncols; c++) out[i * stride + c] = 0.0f;
+    for (int k = 0; k < 3; k++)
+        if (Z.out[k])
+            for (int c = 0; c < Z.cols[k]; c++) Z.out[k][i * Z.stride[k] + c] = 0.0f;
+}
+void zero_unbinned(Volume *v, int64_t n, const ZeroOuts &Z) {
+    const int64_t m = v->res(0) / kCell, nreg = v->atlas_last * m * m * m * kRegions;
+    k_zero_unbinned<<<grid_for(n, 256, 1ll << 31), 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n,
+                                                                        v->reg_off.as<uint32_t>() + nreg, Z);
 }
 
 AtlasGeom atlas_geom(const Volume *v) {
@@ -2299,6 +2314,7 @@ gvdb2_status launch_smem(Volume *v, K kernel, size_t smem, const char *what) {
 template <int NCH>
 __global__ void k_pack_amounts(SplatArgs S) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j == 0) *S.merge_cnt = 0; // for the kernels that follow
     if (j >= (int64_t)S.reg_off[S.ncell * kRegions]) return;
     const int32_t p = S.perm[j];
     if (!in_range(S.lim, p, S.lim.nentry, 11)) {
@@ -2352,7 +2368,7 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     S.merge_cnt = reinterpret_cast<uint32_t *>(v->merge_list.as<char>() + v->merge_list.bytes - 16);
     S.merge_list = v->merge_list.as<int32_t>();
     S.owner_list = v->cell_owner.as<int32_t>();
-    GV_CUDA(v, cudaMemsetAsync(S.merge_cnt, 0, sizeof(uint32_t), v->stream));
+    if (v->bin_key.n == 0) GV_CUDA(v, cudaMemsetAsync(S.merge_cnt, 0, sizeof(uint32_t), v->stream));
     if (v->bin_key.n > 0)
         k_pack_amounts<NCH><<<grid_for(v->bin_key.n, 256, 1ll << 31), 256, 0, v->stream>>>(S);
     if constexpr (KERNEL == GVDB2_KERNEL_CUBIC2) {
@@ -2605,7 +2621,7 @@ gvdb2_status gather_kernel(Volume *v, int kernel, int n, const float trans[3], c
     if (!out || out_stride < nch) return fail(v, GVDB2_ERR_ARG, "bad output buffer");
     GV_TRY(splat_prologue(v, kernel, n, trans));
     if (n == 0) return GVDB2_OK;
-    k_zero_unbinned<<<grid_for(n, 256, 1ll << 31), 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n, out, out_stride, nch);
+    zero_unbinned(v, n, ZeroOuts{{out, nullptr, nullptr}, {out_stride, 0, 0}, {nch, 0, 0}});
     GatherArgs G{};
     G.pos = v->pos;
     G.trans = make_float3(trans[0], trans[1], trans[2]);
@@ -2646,10 +2662,7 @@ gvdb2_status scatter_kernel_backward(Volume *v, int kernel, int n, const float t
     GV_TRY(check_chans(v, grad_chans, nch));
     GV_TRY(splat_prologue(v, kernel, n, trans));
     if (n == 0) return GVDB2_OK;
-    int g = grid_for(n, 256, 1ll << 31);
-    k_zero_unbinned<<<g, 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n, grad_pos, 3, 3);
-    k_zero_unbinned<<<g, 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n, grad_weight, 1, 1);
-    k_zero_unbinned<<<g, 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n, grad_attr, nch, nch);
+    zero_unbinned(v, n, ZeroOuts{{grad_pos, grad_weight, grad_attr}, {3, 1, nch}, {3, 1, nch}});
     GatherArgs G{};
     G.pos = v->pos;
     G.trans = make_float3(trans[0], trans[1], trans[2]);
@@ -2701,7 +2714,7 @@ gvdb2_status gather_kernel_backward(Volume *v, int kernel, int n, const float tr
         GV_TRY(run_scatter(v, kernel, S));
     }
     if (!grad_pos || n == 0) return GVDB2_OK;
-    k_zero_unbinned<<<grid_for(n, 256, 1ll << 31), 256, 0, v->stream>>>(v->pbin.as<int32_t>(), n, grad_pos, 3, 3);
+    zero_unbinned(v, n, ZeroOuts{{grad_pos, nullptr, nullptr}, {3, 0, 0}, {3, 0, 0}});
     GatherArgs G{};
     G.pos = v->pos;
     G.trans = make_float3(trans[0], trans[1], trans[2]);

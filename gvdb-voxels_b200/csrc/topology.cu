@@ -34,7 +34,8 @@ struct SmallWords { // layout of Volume::dev_small
     int32_t splat_guard[5]; // a splat kernel's failed index check: code, index (hi, lo), bound (hi, lo)
     int32_t pad[12];
 };
-static_assert(sizeof(SmallWords) == 128, "small word block");
+static_assert(sizeof(SmallWords) == 128 && sizeof(SmallWords) + sizeof(uint32_t) * kCntWords <= kHostSmallBytes,
+              "small word block, and room for its mirror and the cell counts'");
 
 __device__ __forceinline__ int32_t f2ord(float f) {
     int32_t i = __float_as_int(f);
@@ -45,6 +46,12 @@ inline float ord2f(int32_t o) {
     float f;
     std::memcpy(&f, &i, 4);
     return f;
+}
+
+// An empty bounding box.  (A copy of six words from pageable memory holds the
+// host up longer than this launch.)
+__global__ void k_bbox_init(int32_t *bbox) {
+    if (threadIdx.x < 6) bbox[threadIdx.x] = threadIdx.x < 3 ? f2ord(INFINITY) : f2ord(-INFINITY);
 }
 
 // GetBoundingBox (V:5404-5467): min/max of pos + trans over all points.
@@ -204,19 +211,33 @@ __global__ void k_compact_flagged(const uint64_t *in, int64_t n, const uint32_t 
     if (flags[i]) out[scan[i]] = in[i];
 }
 
-// The root node (V:1290-1300): level `depth`, flags 1, child list Elem(1,depth,0).
-__global__ void k_root(Node *root, int depth, int3 rootpos) {
-    Node nd;
-    memset(&nd, 0, sizeof(nd));
-    nd.mLev = (uint8_t)depth;
-    nd.mFlags = 1;
-    nd.mPos[0] = rootpos.x;
-    nd.mPos[1] = rootpos.y;
-    nd.mPos[2] = rootpos.z;
-    nd.mValue[0] = nd.mValue[1] = nd.mValue[2] = -1;
-    nd.mParent = kUndefL;
-    nd.mChildList = elem(1, depth, 0);
-    *root = nd;
+// The root node (V:1290-1300): level `depth`, flags 1, child list Elem(1,depth,0);
+// the status word cleared; and `n` buffers (child lists, the leaf map's keys)
+// filled with 0xFF, in one launch instead of up to eight.
+struct FillBufs {
+    uint4 *p[kMaxLev + 1];
+    int64_t n16[kMaxLev + 1]; // 16-byte words
+    int n;
+};
+__global__ void k_root_fill(Node *root, int depth, int3 rootpos, int32_t *status, FillBufs F) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        Node nd;
+        memset(&nd, 0, sizeof(nd));
+        nd.mLev = (uint8_t)depth;
+        nd.mFlags = 1;
+        nd.mPos[0] = rootpos.x;
+        nd.mPos[1] = rootpos.y;
+        nd.mPos[2] = rootpos.z;
+        nd.mValue[0] = nd.mValue[1] = nd.mValue[2] = -1;
+        nd.mParent = kUndefL;
+        nd.mChildList = elem(1, depth, 0);
+        *root = nd;
+        *status = 0;
+    }
+    const uint4 ff = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int b = 0; b < F.n; b++)
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < F.n16[b]; i += (int64_t)gridDim.x * blockDim.x)
+            F.p[b][i] = ff;
 }
 
 struct LevelBuild {
@@ -239,11 +260,21 @@ struct LevelBuild {
 // SetupNode (V:2512-2524) for every node of one level, then the link of
 // gvdbLinkBricks (N:470-505): mParent = Elem(0,lev+1,pid) and the parent's
 // child slot (z*res+y)*res+x = Elem(0,lev,i).  Parents are found by key in
-// the parent level's sorted arrays, which is the node getParent reaches.
-__global__ void k_build_link(LevelBuild L) {
-    int64_t n = L.nbase + L.nextra;
+// the parent level's sorted arrays, which is the node getParent reaches.  Every
+// level in one launch, level l's nodes from thread first[l] on: a level reads the
+// key arrays and writes its own nodes and child-list entries only.
+struct LevelBuilds {
+    LevelBuild lev[kMaxLev];
+    int64_t first[kMaxLev + 1];
+    int n;
+};
+__global__ void k_build_link(const __grid_constant__ LevelBuilds A) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= A.first[A.n]) return;
+    int l = 0;
+    while (i >= A.first[l + 1]) l++;
+    const LevelBuild &L = A.lev[l];
+    i -= A.first[l];
     uint64_t key = i < L.nbase ? L.base[i] : L.extra[i - L.nbase];
     int x, y, z;
     unpack_key(key, L.b, x, y, z);
@@ -330,11 +361,11 @@ __global__ void k_atlas_assign(Node *leaves, int64_t n, const uint32_t *flags, c
                                int tile, int apron, AtlasNode *amap, int32_t *slot_leaf, int32_t *leaf_slot) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (!flags[i]) {
+    if (flags && !flags[i]) {
         leaf_slot[i] = -1; // stale leaf keeps its old mValue, as in the reference
         return;
     }
-    int64_t s = slot[i];
+    int64_t s = flags ? slot[i] : i; // no flags: every leaf is flagged
     int64_t a2 = (int64_t)sx * sy;
     int bz = (int)(s / a2);
     int64_t r = s - (int64_t)bz * a2;
@@ -408,7 +439,7 @@ gvdb2_status ensure_small_words(Volume *v) {
         GV_CUDA(v, v->dev_small.ensure(sizeof(SmallWords), v->stream));
         GV_CUDA(v, cudaMemsetAsync(v->dev_small.p, 0, sizeof(SmallWords), v->stream));
     }
-    if (!v->host_small) GV_CUDA(v, cudaMallocHost(&v->host_small, sizeof(SmallWords)));
+    if (!v->host_small) GV_CUDA(v, cudaMallocHost(&v->host_small, kHostSmallBytes));
     return GVDB2_OK;
 }
 
@@ -634,26 +665,35 @@ gvdb2_status build_from_keys(Volume *v, const int64_t nB[], const int64_t nE[], 
     for (int l = 0; l < kMaxLev; l++) v->pool_cnt[l] = 0;
     for (int l = 0; l < depth; l++) v->pool_cnt[l] = nB[l] + nE[l];
     v->pool_cnt[depth] = 1;
+    FillBufs F{};
+    auto fill = [&](void *p, size_t bytes) { // allocations and their sizes are whole 16-byte words
+        F.p[F.n] = static_cast<uint4 *>(p);
+        F.n16[F.n++] = (int64_t)(bytes / 16);
+    };
     for (int l = 0; l <= depth; l++) {
         GV_TRY(ensure_pool(v, l, v->pool_cnt[l]));
         v->lev_count[l][0] = nB[l];
         v->lev_count[l][1] = nE[l];
-        if (l > 0)
-            GV_CUDA(v, cudaMemsetAsync(v->clist[l].p, 0xFF, sizeof(uint64_t) * (size_t)(v->pool_cnt[l] * v->res3(l)), s));
+        if (l > 0) fill(v->clist[l].p, sizeof(uint64_t) * (size_t)(v->pool_cnt[l] * v->res3(l))); // res3 >= 8
     }
-    k_root<<<1, 1, 0, s>>>(v->pool_ptr(depth), depth, make_int3(v->root_pos[0], v->root_pos[1], v->root_pos[2]));
 
     // leaf map: level-0 key -> pool index
     uint32_t lcap = next_pow2((uint64_t)std::max<int64_t>(2 * v->pool_cnt[0], 1 << 12));
     GV_CUDA(v, v->leafmap_keys.ensure(sizeof(uint64_t) * lcap, s));
     GV_CUDA(v, v->leafmap_vals.ensure(sizeof(int32_t) * lcap, s));
-    GV_CUDA(v, cudaMemsetAsync(v->leafmap_keys.p, 0xFF, sizeof(uint64_t) * lcap, s));
+    fill(v->leafmap_keys.p, sizeof(uint64_t) * lcap);
     v->leafmap_mask = lcap - 1;
     v->leafmap_is_tree = true;
-    GV_CUDA(v, cudaMemsetAsync(&dev_words(v)->status, 0, sizeof(int32_t), s));
+    int64_t words = 0;
+    for (int b = 0; b < F.n; b++) words += F.n16[b];
+    k_root_fill<<<grid_for(words, 256, 8 * kSmCount), 256, 0, s>>>(
+        v->pool_ptr(depth), depth, make_int3(v->root_pos[0], v->root_pos[1], v->root_pos[2]), &dev_words(v)->status, F);
 
+    LevelBuilds A;
+    A.n = depth;
+    A.first[0] = 0;
     for (int l = 0; l < depth; l++) {
-        LevelBuild L;
+        LevelBuild &L = A.lev[l];
         L.base = v->lev_keys[l][0].as<uint64_t>();
         L.nbase = nB[l];
         L.extra = v->lev_keys[l][1].as<uint64_t>();
@@ -676,10 +716,10 @@ gvdb2_status build_from_keys(Volume *v, const int64_t nB[], const int64_t nE[], 
         L.leaf_vals = v->leafmap_vals.as<int32_t>();
         L.leaf_mask = v->leafmap_mask;
         L.status = &dev_words(v)->status;
-        int64_t cnt = nB[l] + nE[l];
-        if (cnt > 0) k_build_link<<<grid_for(cnt, 256, 1ll << 31), 256, 0, s>>>(L);
-        GV_CUDA(v, cudaGetLastError());
+        A.first[l + 1] = A.first[l] + nB[l] + nE[l];
     }
+    if (A.first[depth] > 0) k_build_link<<<grid_for(A.first[depth], 256, 1ll << 31), 256, 0, s>>>(A);
+    GV_CUDA(v, cudaGetLastError());
     // the status word is checked at the next read-back of the small words
     // (the next rebuild's bounding box, Synchronize or GetInfo), not by a
     // stall here
@@ -1263,9 +1303,19 @@ KeyGeom key_geom(const Volume *v) {
 
 gvdb2_status incremental_rebuild(Volume *v, int n, float radius, const float orig[3], bool accum);
 
-gvdb2_status flush_status(Volume *v) {
-    if (!(v->status_pending || v->splat_guard_pending) || !v->dev_small.p) return GVDB2_OK;
-    return read_words(v);
+gvdb2_status flush_status(Volume *v, int64_t *cells) {
+    // the bins' cell counts come with the words, once per binning
+    const bool bins = cells && v->bin_key.valid && v->cell_cnt.p && v->host_small;
+    uint32_t *c3 = reinterpret_cast<uint32_t *>(static_cast<char *>(v->host_small) + sizeof(SmallWords));
+    const bool fetch = bins && !v->cells_read;
+    if (fetch)
+        GV_CUDA(v, cudaMemcpyAsync(c3, v->cell_cnt.p, sizeof(uint32_t) * kCntWords, cudaMemcpyDeviceToHost, v->stream));
+    gvdb2_status st = GVDB2_OK;
+    if ((v->status_pending || v->splat_guard_pending) && v->dev_small.p) st = read_words(v);
+    else if (fetch) GV_CUDA(v, cudaStreamSynchronize(v->stream));
+    if (fetch) v->cells_read = true;
+    if (bins) *cells = (int64_t)c3[kCntHuge] + c3[kCntHeavy] + c3[kCntLight];
+    return st;
 }
 
 int32_t *splat_guard_word(Volume *v) { return v->dev_small.p ? dev_words(v)->splat_guard : nullptr; }
@@ -1329,12 +1379,7 @@ gvdb2_status rebuild_topology(Volume *v, int n, float radius, const float orig[3
     GV_TRY(ensure_small_words(v));
     reserve_pool(v, n);
     // GetBoundingBox
-    int32_t init[6];
-    for (int a = 0; a < 3; a++) {
-        init[a] = 0x7F800000;            // ord(+inf)
-        init[3 + a] = (int32_t)0x807FFFFF; // ord(-inf)
-    }
-    GV_CUDA(v, cudaMemcpyAsync(dev_words(v)->bbox, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_bbox_init<<<1, 32, 0, s>>>(dev_words(v)->bbox);
     if (n > 0)
         k_bbox<<<std::min(grid_for(n, 256), 8 * kSmCount), 256, 0, s>>>(v->pos, n, make_float3(orig[0], orig[1], orig[2]),
                                                                         dev_words(v)->bbox);
@@ -1416,18 +1461,19 @@ gvdb2_status update_atlas(Volume *v) {
     cudaStream_t s = v->stream;
     int64_t total = v->pool_cnt[0];
     v->atlas_last = 0;
-    uint32_t *flags = nullptr;
-    GV_CUDA(v, cudaMallocAsync((void **)&flags, sizeof(uint32_t) * (size_t)(2 * total + 2), s));
-    uint32_t *scan = flags + total + 1;
-    if (total > 0) k_leaf_flags<<<grid_for(total, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), total, flags);
-    gvdb2_status st = exclusive_scan_u32(v, flags, scan, total);
-    uint32_t nflag = 0;
-    if (st == GVDB2_OK && v->all_leaves_flagged) {
-        nflag = (uint32_t)total; // a full rebuild flags every leaf: no read-back
-    } else if (st == GVDB2_OK) {
-        cudaError_t e = cudaMemcpyAsync(&nflag, scan + total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) st = cuda_fail(v, e, "update_atlas count");
+    uint32_t *flags = nullptr, *scan = nullptr;
+    gvdb2_status st = GVDB2_OK;
+    uint32_t nflag = (uint32_t)total; // a full rebuild flags every leaf: slots are pool indices
+    if (!v->all_leaves_flagged) {
+        GV_CUDA(v, cudaMallocAsync((void **)&flags, sizeof(uint32_t) * (size_t)(2 * total + 2), s));
+        scan = flags + total + 1;
+        if (total > 0) k_leaf_flags<<<grid_for(total, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), total, flags);
+        st = exclusive_scan_u32(v, flags, scan, total);
+        if (st == GVDB2_OK) {
+            cudaError_t e = cudaMemcpyAsync(&nflag, scan + total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess) st = cuda_fail(v, e, "update_atlas count");
+        }
     }
     if (st == GVDB2_OK && (v->used_leaves > v->atlas_cap || (int64_t)nflag > v->atlas_cap))
         st = atlas_resize(v, std::max<int64_t>(v->used_leaves, nflag));
@@ -1435,7 +1481,9 @@ gvdb2_status update_atlas(Volume *v) {
         cudaError_t e = v->amap.ensure(sizeof(AtlasNode) * (size_t)v->atlas_cap, s);
         if (e == cudaSuccess) e = v->slot_leaf.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(v->atlas_cap, 1), s);
         if (e == cudaSuccess) e = v->leaf_slot.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(total, 1), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(v->amap.p, 0xFF, sizeof(AtlasNode) * (size_t)v->atlas_cap, s);
+        // entries past the slots in use
+        if (e == cudaSuccess && (int64_t)nflag < v->atlas_cap)
+            e = cudaMemsetAsync(v->amap.as<AtlasNode>() + nflag, 0xFF, sizeof(AtlasNode) * (size_t)(v->atlas_cap - nflag), s);
         if (e != cudaSuccess) st = cuda_fail(v, e, "update_atlas alloc");
     }
     if (st == GVDB2_OK && total > 0) {
@@ -1445,7 +1493,7 @@ gvdb2_status update_atlas(Volume *v) {
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(v, e, "k_atlas_assign");
     }
-    cudaFreeAsync(flags, s);
+    if (flags) cudaFreeAsync(flags, s);
     if (st != GVDB2_OK) return st;
     v->atlas_last = nflag;
     // 27-neighbour slot table for the splat/apron kernels

@@ -154,3 +154,31 @@ def test_voxel_gathers_list_ends(gvdb2_mod, oracle_mod, levelset, per_list):
         v.GatherDensity(4, len(pts), 1.5, (0, 0, 0), ln, 0)
         o.gather_density(4, 1.5, 0)
     assert rel_err(interior(v.atlas(0), 1), interior(o.atlas(0), 1)) < REL_TOL
+
+
+@pytest.mark.parametrize("outside", [0, 1, 300])
+def test_points_outside_the_bricks(gvdb2_mod, outside):
+    """Gathers and gradients of points outside every brick are zero whatever the buffers held, and the others are those
+    of a call without them (deterministic mode, exactly)."""
+    import torch
+    rng = np.random.default_rng(26)
+    inside = rng.uniform(70.0, 90.0, (1000, 3)).astype(np.float32)
+    pts = np.concatenate([inside, rng.uniform(300.0, 400.0, (outside, 3)).astype(np.float32)])
+    n, res = len(pts), []
+    for p in (inside, pts):
+        v = gpu_volume(gvdb2_mod, inside, chans=[0])
+        v.SetDeterministic(True)
+        v.RebuildTopology(len(inside), 2.0)
+        v.UpdateAtlas()
+        t = torch.from_numpy(p).cuda()
+        v.SetPoints(t)
+        v.ScatterKernel(2, len(p), [0])
+        out = [torch.full(s, float("nan"), device="cuda") for s in ((len(p), 1), (len(p), 3), (len(p),), (len(p), 1), (len(p), 3))]
+        v.GatherKernel(2, len(p), [0], out=out[0])
+        v.ScatterDensityBackward(2, len(p), [0], attrs=[torch.ones(len(p), device="cuda")], grad_pos=out[1],
+                                 grad_weight=out[2], grad_attr=out[3])
+        v.GatherDensityBackward(2, len(p), [0], torch.ones((len(p), 1), device="cuda"), grad_pos=out[4])
+        res.append([o.cpu().numpy() for o in out])
+    for a, b in zip(*res):
+        assert np.array_equal(b[:1000], a)
+        assert not b[1000:n].any()
