@@ -175,14 +175,15 @@ __device__ __forceinline__ void cell_coords(int64_t cell, int m, int m3, int64_t
 }
 // The cells that hold points fall in three classes by their point count k:
 // huge (k > kHeavyCell), heavy (kLightCell < k <= kHeavyCell) and light
-// (0 < k <= kLightCell).  The huge and heavy cells are listed in the order
-// of cell_at: huge cells first (list[0 .. cnt[0])), then the heavy ones,
-// stored from the back (list[ncell - 1], list[ncell - 2], ..., cnt[1] of
-// them).  Light cells are listed apart (light[0 .. cnt[2])).  The gather
-// stages a halo tile per huge or heavy cell and reads the taps of light
-// cells' points straight from the atlas, one warp per light cell.
+// (0 < k <= kLightCell).  Heavy and light cells are listed; a huge cell is listed
+// as items (cell, slice) of kTilePts points.  The gather stages a halo tile per
+// item or heavy cell and reads the taps of light cells' points straight from the
+// atlas, four light cells a warp.  A CTA a huge cell made the largest the launch's
+// tail: a scene whose densest cells hold 130,000 points gathered 3 and 4 channels
+// forward and back in 1.92 + 2.02 + 3.45 ms, with items in 1.47 + 1.94 + 3.16.
 constexpr uint32_t kHeavyCell = 1024;
 constexpr uint32_t kLightCell = 32;
+constexpr uint32_t kTilePts = 2048;
 // Cells of at least kDenseCell points are splatted into partial sums (the
 // scatter's dense path), kSlicePts points per CTA.
 #ifndef GVDB2_DENSE_CELL
@@ -213,9 +214,9 @@ __device__ __forceinline__ bool in_range(const SplatLimits &L, int64_t i, int64_
 constexpr uint32_t kSlicePts = 4096;
 // cell_cnt entries: huge, heavy, light cells; dense cells, dense work
 // items (slices), dense cells of more than one slice, cells listed for
-// k_scatter_cells, dense cells listed for k_scatter_rows
+// k_scatter_cells, dense cells listed for k_scatter_rows, items of huge cells
 constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntOwner = 6,
-              kCntRows = 7, kCntWords = 8;
+              kCntRows = 7, kCntTiles = 8, kCntWords = 12;
 // Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic): 16.7M
 // points in cells of 1,024 on average, 4 channels, 1.22 + 0.13 ms (its sort)
 // against 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162
@@ -243,13 +244,6 @@ static_assert(kRowsMax <= 65535, "16-bit positions in a cell");
 #endif
 constexpr int32_t kPartListed = -2; // a cell's partial slot when it is listed for k_scatter_cells
 constexpr int kLightOwn = GVDB2_LIGHT_OWN, kHeavyFace = GVDB2_HEAVY_FACE;
-// The i-th huge or heavy cell, or -1 past their end.
-__device__ __forceinline__ int64_t cell_at(int64_t i, const int32_t *list, const uint32_t *cnt, int64_t ncell) {
-    const int64_t h = cnt[0];
-    if (i < h) return list[i];
-    i -= h;
-    return i < (int64_t)cnt[1] ? list[ncell - 1 - i] : -1;
-}
 // cell of a voxel inside its brick (local voxel coordinates in [0, res0))
 __device__ __forceinline__ int cell_of_local(int lx, int ly, int lz, int m) {
     return ((lz >> 3) * m + (ly >> 3)) * m + (lx >> 3);

@@ -210,11 +210,11 @@ struct Volume {
     DevBuf rows_list, row_off;
     int64_t rows_cap = 0;
     bool rows_sorted = false;
-    // cells that hold points: huge and heavy ones (order of cell_at), light
-    // ones and the counts (kCnt*); heavy_grid, light_grid and cell_grid
-    // bound the huge+heavy, light and all lists
-    DevBuf cell_list, cell_light, cell_cnt;
-    int64_t cell_grid = 0, heavy_grid = 0, light_grid = 0;
+    // cells that hold points: heavy ones, light ones, items (cell, slice) of huge
+    // ones, and the counts (kCnt*); heavy_grid and light_grid bound items + heavy
+    // cells and light cells
+    DevBuf cell_list, cell_light, cell_tiles, cell_cnt;
+    int64_t heavy_grid = 0, light_grid = 0;
     struct BinKey {
         bool valid = false;
         int kernel = 0;

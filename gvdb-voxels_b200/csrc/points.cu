@@ -140,8 +140,8 @@ __global__ void k_bin_pack_pos(const int32_t *perm, const uint32_t *reg_off, int
     bin_pos[j] = make_float4(q.x + trans.x, q.y + trans.y, q.z + trans.z, __int_as_float(cloud));
 }
 
-// List the cells that hold points by class (huge from the front of `list`,
-// heavy from its back, light in `light`; see cell_at).
+// List the cells that hold points by class: heavy in `list`, light in `light`, huge
+// as items (cell, slice) in `tiles`.
 constexpr int64_t kCellCountReadback = 1 << 16; // cells
 
 // Cells of at least `dense_min` points (dense_min > 0) are the scatter's dense
@@ -156,7 +156,8 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // volume of its own gets.
 // reg_off holds each (cell, region) bin's first entry; off[c] = reg_off[27 c], each
 // cell's (c = ncell: the end), is written for the kernels that follow.
-__global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int32_t *part,
+__global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int2 *tiles,
+                            int32_t *part,
                             int32_t *owner, int32_t *rows, int4 *work, uint32_t *cnt, const int32_t *nbr27, int m,
                             uint32_t dense_min,
                             uint32_t slice, uint32_t light_max, bool cubic, bool rows_on) {
@@ -169,7 +170,11 @@ __global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncel
     if (cls >= 0) {
         const uint32_t r = warp_agg_inc(cnt, (uint32_t)cls, act);
         if (cls == kCntLight) light[r] = (int32_t)c;
-        else list[cls == kCntHuge ? (int64_t)r : ncell - 1 - r] = (int32_t)c;
+        else if (cls == kCntHeavy) list[r] = (int32_t)c;
+        else {
+            const uint32_t ns = (k + kTilePts - 1) / kTilePts, t = atomicAdd(cnt + kCntTiles, ns);
+            for (uint32_t i = 0; i < ns; i++) tiles[t + i] = make_int2((int32_t)c, (int32_t)i);
+        }
     }
     const bool dense = dense_min > 0 && k >= dense_min;
     const unsigned dn = __ballot_sync(0xffffffffu, dense);
@@ -483,6 +488,8 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     // scatter's dense cells with their work items
     GV_CUDA(v, v->cell_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     GV_CUDA(v, v->cell_light.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
+    // an item a huge cell, and one more for each kTilePts of its points
+    GV_CUDA(v, v->cell_tiles.ensure(sizeof(int2) * (size_t)(n / (kHeavyCell + 1) + n / kTilePts + 1), s));
     GV_CUDA(v, v->cell_part.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     GV_CUDA(v, v->cell_owner.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(nbins, 1), s));
     // bounds from the point count: at most n / dense dense cells, and each
@@ -498,27 +505,28 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     v->multi_cap = std::min<int64_t>(v->dense_cap, n / (sl + 1));
     GV_CUDA(v, v->rows_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(v->rows_cap, 1), s));
     GV_CUDA(v, v->part_work.ensure(sizeof(int4) * (size_t)std::max<int64_t>(v->work_cap, 1), s));
-    v->cell_grid = v->heavy_grid = v->light_grid = 0;
+    v->heavy_grid = v->light_grid = 0;
     v->cells_read = false;
     if (nbins == 0) GV_CUDA(v, cudaMemsetAsync(v->bin_off.p, 0, sizeof(uint32_t), s));
     if (nbins > 0) {
         const int g = grid_for(nbins + 1, 256, 1ll << 31);
         k_cell_list<<<g, 256, 0, s>>>(v->reg_off.as<uint32_t>(), v->bin_off.as<uint32_t>(), nbins, v->cell_list.as<int32_t>(),
-                                      v->cell_light.as<int32_t>(), v->cell_part.as<int32_t>(), v->cell_owner.as<int32_t>(),
+                                      v->cell_light.as<int32_t>(), v->cell_tiles.as<int2>(),
+                                      v->cell_part.as<int32_t>(), v->cell_owner.as<int32_t>(),
                                       v->rows_list.as<int32_t>(), v->part_work.as<int4>(), v->cell_cnt.as<uint32_t>(),
                                       v->nbr27.as<int32_t>(), m, (uint32_t)dmin, (uint32_t)v->tune_slice, (uint32_t)v->tune_light,
                                       cubic, rows);
         GV_CUDA(v, cudaGetLastError());
-        v->cell_grid = v->heavy_grid = v->light_grid = nbins;
+        v->heavy_grid = nbins + n / kTilePts;
+        v->light_grid = nbins;
         if (nbins > kCellCountReadback) {
             // many cells: size the grids by the cells of each class (one
-            // 32-byte read) rather than by all cells
+            // small read) rather than by all cells
             uint32_t cw[kCntWords] = {0};
             GV_CUDA(v, cudaMemcpyAsync(cw, v->cell_cnt.p, sizeof(cw), cudaMemcpyDeviceToHost, s));
             GV_CUDA(v, cudaStreamSynchronize(s));
-            v->heavy_grid = (int64_t)cw[kCntHuge] + cw[kCntHeavy];
+            v->heavy_grid = (int64_t)cw[kCntTiles] + cw[kCntHeavy];
             v->light_grid = cw[kCntLight];
-            v->cell_grid = v->heavy_grid + v->light_grid;
             v->dense_cap = cw[kCntDense];
             v->rows_cap = cw[kCntRows];
             v->work_cap = cw[kCntWork];

@@ -219,9 +219,8 @@ struct SplatArgs {
     float4 *bin_amt;         // per entry of perm: the channel amounts of this call
     int res0, apron, tile;
     int m, m3; // cells per brick edge, per brick
-    // huge and heavy cells (order of cell_at), light cells; cell_list ==
-    // nullptr: every cell, in cell order
-    const int32_t *cell_list, *cell_light;
+    const int32_t *cell_list, *cell_light; // heavy, light cells
+    const int2 *cell_tiles;                // items of huge cells
     const uint32_t *cell_cnt;
     int64_t ncell;
     int64_t tvox;
@@ -1835,9 +1834,8 @@ struct GatherArgs {
     const int32_t *perm;
     int res0, apron, tile;
     int m, m3; // cells per brick edge, per brick
-    // huge and heavy cells (order of cell_at), light cells; cell_list ==
-    // nullptr: every cell, in cell order
-    const int32_t *cell_list, *cell_light;
+    const int32_t *cell_list, *cell_light; // heavy, light cells; cell_list == nullptr: every cell, in cell order
+    const int2 *cell_tiles;                // items of huge cells
     const uint32_t *cell_cnt;
     int64_t ncell;
     int64_t tvox;
@@ -1990,8 +1988,8 @@ constexpr size_t gather_tile_smem() {
            sizeof(uint32_t) * 1024;
 }
 
-// One CTA per huge or heavy cell (every cell when the binning came from the
-// caller): stages the cell plus a halo of N/2 voxels (12^3 for the cubic
+// One CTA per heavy cell or item of a huge one (per cell when the binning came
+// from the caller): stages the cell plus a halo of N/2 voxels (12^3 for the cubic
 // B-spline) from the interiors of its brick and the neighbours, the
 // channels of a voxel side by side, then serves the cell's points from
 // shared memory.  The points are visited in the order of their first tap
@@ -2013,10 +2011,25 @@ __device__ __forceinline__ void gather_tile_cell(const GatherArgs &G, int64_t bl
     __shared__ int32_t nbs[27];
     __shared__ uint32_t wsum[kGatherThreads / 32];
     const int res = G.res0;
-    const int64_t cell = G.cell_list ? cell_at(block, G.cell_list, G.cell_cnt, G.ncell) : block;
-    if (cell < 0) return;
-    const uint32_t beg = G.bin_off[cell], end = G.bin_off[cell + 1];
-    if (beg == end) return; // no points: nothing to stage
+    int64_t cell = block;
+    uint32_t first = 0, most = UINT32_MAX; // the cell's points [first, first + most)
+    if (G.cell_list) {
+        const int64_t items = G.cell_cnt[kCntTiles];
+        if (block < items) {
+            const int2 t = G.cell_tiles[block];
+            cell = t.x;
+            first = (uint32_t)t.y * kTilePts;
+            most = kTilePts;
+        } else {
+            if (block - items >= (int64_t)G.cell_cnt[kCntHeavy]) return;
+            cell = G.cell_list[block - items];
+        }
+        if (!in_range(G.lim, cell, G.ncell, 41)) return;
+    }
+    const uint32_t beg = G.bin_off[cell] + first;
+    uint32_t end = G.bin_off[cell + 1];
+    if (beg >= end) return; // no points: nothing to stage
+    end = min(end - beg, most) + beg;
     int64_t slot;
     int cx, cy, cz;
     cell_coords(cell, G.m, G.m3, slot, cx, cy, cz);
@@ -2222,7 +2235,7 @@ __device__ __forceinline__ void gather_light_cells(const GatherArgs &G, int64_t 
     }
 }
 
-// Two launches: a halo tile per huge or heavy cell (every cell, in cell
+// Two launches: a halo tile per item or heavy cell (every cell, in cell
 // order, when no cell list is given), then the light cells, kLightPack a warp.
 // One fused launch measured slower: the light path's registers (66) halved
 // the tiles' occupancy.
@@ -2284,6 +2297,7 @@ void fill_topology(Volume *v, Args &S) {
     S.m = v->res(0) / kCell;
     S.m3 = S.m * S.m * S.m;
     S.cell_list = v->cell_list.as<int32_t>();
+    S.cell_tiles = v->cell_tiles.as<int2>();
     S.cell_light = v->cell_light.as<int32_t>();
     S.cell_cnt = v->cell_cnt.as<uint32_t>();
     S.ncell = v->atlas_last * S.m3;
@@ -2467,7 +2481,7 @@ gvdb2_status launch_gather(Volume *v, const GatherArgs &G) {
     constexpr size_t smem = gather_tile_smem<KERNEL, NCH>();
     auto k = k_gather_tile<KERNEL, MODE, NCH>;
     GV_TRY(launch_smem(v, k, smem, "gather"));
-    // tiles for the huge and heavy cells, then the light cells, a warp each
+    // tiles for the huge cells' items and the heavy cells, then the light cells
     // (every cell gets a tile when the caller supplied the binning)
     const int64_t heavy = G.cell_list ? v->heavy_grid : G.ncell;
     if (heavy > 0) k<<<(unsigned)heavy, kGatherThreads, smem, v->stream>>>(G);

@@ -182,3 +182,28 @@ def test_points_outside_the_bricks(gvdb2_mod, outside):
     for a, b in zip(*res):
         assert np.array_equal(b[:1000], a)
         assert not b[1000:n].any()
+
+
+@pytest.mark.parametrize("per_cell", [1024, 1025, 2048, 2049, 4097])
+def test_gather_huge_cells(gvdb2_mod, oracle_mod, per_cell):
+    """A cell at the ends of the heavy class and of the gather's items of 2,048 points: gather and both adjoints against
+    the FP64 oracle within 1e-5 of the largest value, every point served."""
+    import torch
+    rng = np.random.default_rng(27)
+    pts = rng.uniform(80.0, 87.99, (per_cell, 3)).astype(np.float32)
+    n = len(pts)
+    o = make_oracle(oracle_mod, chans=[0])
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.update_atlas()
+    v = gpu_volume(gvdb2_mod, pts, chans=[0])
+    v.RebuildTopology(n, 2.0)
+    v.UpdateAtlas()
+    assert v.info().splat_cells == -1
+    v.ScatterKernel(2, n, [0])
+    o.scatter_kernel(2, pts, [0])
+    assert v.info().splat_cells == 1
+    out = torch.full((n, 1), float("nan"), device="cuda")
+    assert rel_err(v.GatherKernel(2, n, [0], out=out).cpu().numpy(), o.gather_kernel(2, pts, [0])) < REL_TOL
+    go = rng.normal(size=(n, 1)).astype(np.float32)
+    gp = v.GatherDensityBackward(2, n, [0], torch.from_numpy(go).cuda()).cpu().numpy()
+    assert rel_err(gp, o.gather_kernel_backward(2, pts, [0], go)) < REL_TOL
