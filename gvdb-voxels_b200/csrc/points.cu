@@ -3,7 +3,7 @@
 //   InsertPoints (V:5219-5267, P:19-36, P:59-72): per point the leaf it
 //     falls in (pnode), its slot inside that leaf (poff) and per-leaf
 //     counts (gcnt); with `prefix`, a counting sort of positions by leaf.
-//   Kernel-splat binning (no reference counterpart): a warp-aggregated
+//   Kernel-splat binning (no reference counterpart): a
 //     counting sort of points by (atlas slot, region) where the 27 regions
 //     say which neighbouring bricks a point's stencil reaches; the splat
 //     kernels read a brick's own points plus the matching regions of its
@@ -58,8 +58,10 @@ __global__ void k_sort_points(PointsView pos, int64_t n, float3 trans, const int
 // tap < 0), 2 when it reaches into the cell above (last tap >= 8), else 1 (a
 // stencil is narrower than a cell, so never both).  A cell's points so come
 // ordered by region, and the points of a neighbour whose stencils reach a
-// cell are a few contiguous runs of that neighbour's bin.  Ranks come from
-// warp-aggregated counters.
+// cell are a few contiguous runs of that neighbour's bin.  Bound by the latency
+// of the leaf lookup and by an atomic add a point.  (One add for the points of a
+// warp that share a bin: 16.7M lattice points 201 us against 176, 1M shell points
+// 28 against 17, 16.7M points in random order 393 against 355.)
 template <int KERNEL>
 __device__ __forceinline__ int region_axis(float w, int cell_lo) {
     // first tap of Taps<KERNEL>::eval, relative to the cell's first voxel
@@ -92,11 +94,9 @@ __global__ void k_bin_count(PointsView pos, int64_t n, float3 trans, LeafLookup 
             }
         }
     }
-    unsigned act = __ballot_sync(0xffffffffu, bin >= 0);
     if (bin >= 0) {
-        uint32_t r = warp_agg_inc(cnt, (uint32_t)bin, act);
         pbin[i] = bin;
-        prank[i] = (int32_t)r;
+        prank[i] = (int32_t)atomicAdd(cnt + bin, 1u);
     } else if (i < n) {
         pbin[i] = -1;
     }

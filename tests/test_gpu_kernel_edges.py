@@ -190,7 +190,7 @@ def test_gather_huge_cells(gvdb2_mod, oracle_mod, per_cell):
     the FP64 oracle within 1e-5 of the largest value, every point served."""
     import torch
     rng = np.random.default_rng(27)
-    pts = rng.uniform(80.0, 87.99, (per_cell, 3)).astype(np.float32)
+    pts = np.concatenate([rng.uniform(80.0, 87.99, (per_cell, 3)), [[100.0, 100.0, 100.0]]]).astype(np.float32)
     n = len(pts)
     o = make_oracle(oracle_mod, chans=[0])
     assert o.rebuild_topology(pts, 2.0) == 0
@@ -201,7 +201,7 @@ def test_gather_huge_cells(gvdb2_mod, oracle_mod, per_cell):
     assert v.info().splat_cells == -1
     v.ScatterKernel(2, n, [0])
     o.scatter_kernel(2, pts, [0])
-    assert v.info().splat_cells == 1
+    assert v.info().splat_cells == 2
     out = torch.full((n, 1), float("nan"), device="cuda")
     assert rel_err(v.GatherKernel(2, n, [0], out=out).cpu().numpy(), o.gather_kernel(2, pts, [0])) < REL_TOL
     go = rng.normal(size=(n, 1)).astype(np.float32)
