@@ -626,13 +626,14 @@ __device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *
 // z0: lane (y, z) holds target row y of the half's 8 and target plane z0 + z,
 // and keeps the 4 columns a stencil covers in registers, a window that moves
 // along x; a column that the window leaves is added to the half's planes in
-// shared memory, which hold 5 planes in turn.  After plane z0's last unit its
+// shared memory, which hold 4 planes in turn.  After plane z0's last unit its
 // rows, the two halves' sums together, go to the partial.
 //
 // Per point and channel pair a lane adds 4 products (packed FMAs), half of
 // them zero (4 of the 8 rows): bound by instruction issue and by the latency
-// of the records' reads (43% of issue slots, 14 warps an SM: shared memory for
-// 24 KB a cell).  The fixed-point atomics of k_scatter_part, two per tap and
+// of the records' reads (43% of issue slots with 14 warps an SM; shared memory
+// for 20 KB a cell bounds them: with a fifth plane, which spares a barrier a
+// plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points).  The fixed-point atomics of k_scatter_part, two per tap and
 // channel, are bound by the shared-memory atomic rate, 30 of 32 lanes a cycle.
 //
 // Sums are float, at most some 20 terms in a register window, then up to 8
@@ -735,12 +736,12 @@ struct PartPos {
 };
 __device__ constexpr PartPos kPartPos{};
 
-constexpr int kRowRec = 28; // floats a record: x weights twice each, 8 y weights, z weights, amounts, padding
+constexpr int kRowRec = 24; // floats a record: x weights twice each, 8 y weights, z weights, amounts
 template <int NCH>
 struct RowSmem {
     // [half][plane in turn][row][column]: the odd row stride and the plane stride
     // of 8 modulo 32 words put a flush's 32 values in different banks
-    typename GVec<NCH>::T plane[2][5][8][13];
+    typename GVec<NCH>::T plane[2][4][8][13];
     float rec[2][32][kRowRec];
     uint16_t off[kRowOff];
 };
@@ -830,13 +831,13 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
     };
     uint32_t i = M.off[half * 81], staged = i; // the points below `staged` are in rec
     fetch(i);
-    int turn = 0; // z0 modulo 5
+    int turn = 0; // z0 modulo 4
     for (int z0 = 0; z0 < X::E; z0++) {
         if (z0 < 9) {
             const uint16_t *off = M.off + (half * 9 + z0) * 9;
             if (off[0] < off[9]) {
                 int t = turn + tz;
-                if (t >= 5) t -= 5;
+                if (t >= 4) t -= 4;
                 V *row = M.plane[half][t][ty];
                 float2 acc[4][NP];
 #pragma unroll
@@ -893,8 +894,7 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
             }
         }
         __syncthreads(); // both halves are done with plane z0
-        // its rows: 0..7 from half 0, 5..11 from half 1; the planes of the next
-        // first plane are other ones, so it may start meanwhile
+        // its rows: 0..7 from half 0, 5..11 from half 1
         for (int v = threadIdx.x; v < X::E * X::E; v += 64) {
             const int y = v / X::E, x = v - y * X::E;
             float sum[4] = {0.f, 0.f, 0.f, 0.f};
@@ -914,7 +914,8 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
 #pragma unroll
             for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] = sum[c];
         }
-        turn = turn == 4 ? 0 : turn + 1;
+        turn = turn == 3 ? 0 : turn + 1;
+        __syncthreads(); // the next units add to this plane's place
     }
 }
 
