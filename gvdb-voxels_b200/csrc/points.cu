@@ -234,7 +234,7 @@ struct ScArgs {
     LeafLookup L;
     const Node *leaves;
     int64_t nleaves;
-    const uint32_t *mapping;
+    const uint32_t *mapping; // a leaf's place among the listed ones (nullptr: its pool index)
     // pass 2 (InsertPointsSubcell_FP16): quantization ranges, velocities
     float3 pmin, prange, vmin, vrange;
     PointsView vel;
@@ -261,8 +261,7 @@ __device__ __forceinline__ uint16_t quantize16(float x, float lo, float range) {
 // 581 us to count and insert.  (Brick by brick, the lanes' loops diverge: 361 +
 // 683.  One add for the lanes of a warp that visit a subcell together: 508 + 938.)
 template <int PASS>
-__global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const uint32_t *off, float *pnt,
-                           int32_t *status) {
+__global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *off, float *pnt) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.n) return;
     float3 p = load_f3(A.pos, i);
@@ -297,15 +296,16 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const u
     // first subcell of a brick's subcells, or -1
     auto first_of = [&](int bx, int by, int bz) {
         const int32_t leaf = leaf_at_brick(A.L, bx, by, bz);
-        return leaf < 0 || leaf >= A.nleaves ? int64_t(-1) : (int64_t)A.mapping[leaf] * A.scpb;
+        if (leaf < 0 || leaf >= A.nleaves) return int64_t(-1);
+        return (int64_t)(A.mapping ? A.mapping[leaf] : (uint32_t)leaf) * A.scpb;
     };
     auto place = [&](int64_t idx, uint32_t o) {
-        if (o >= cap[idx]) {
+        const uint32_t first = off[idx];
+        if (o >= off[idx + 1] - first) {
             atomicSub(&cnt[idx], 1u); // the list keeps its counted length
-            atomicOr(status, kDevCapacity);
             return;
         }
-        const int64_t at = (int64_t)off[idx] + o;
+        const int64_t at = (int64_t)first + o;
         if (PASS == 2) {
             A.q[3 * at + 0] = quantize16(w[0], A.pmin.x, A.prange.x);
             A.q[3 * at + 1] = quantize16(w[1], A.pmin.y, A.prange.y);
@@ -376,7 +376,7 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *cap, const u
 // (scpb subcells a leaf, 512 of them in a 32^3 brick).  Bound by its 16 bytes
 // of stores a subcell; a thread per leaf that looped over its subcells left
 // all but a few warps idle (150 bricks of 32^3: 313 us, 48 bricks: 177 us;
-// a thread per subcell: 3 us).
+// a thread per subcell: 2 us).
 __global__ void k_sc_pos(const Node *leaves, int64_t n, const uint32_t *mapping, int sc, int scdim, int scpb,
                          int64_t num_sc, int32_t *sc_nid, int32_t *sc_pos) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,7 +385,7 @@ __global__ void k_sc_pos(const Node *leaves, int64_t n, const uint32_t *mapping,
     const int s = (int)(t - i * scpb);
     const Node &nd = leaves[i];
     if (nd.mParent == kUndef64) return;
-    const int64_t idx = (int64_t)mapping[i] * scpb + s;
+    const int64_t idx = (mapping ? (int64_t)mapping[i] : i) * scpb + s;
     if (idx >= num_sc) return;
     sc_pos[3 * idx + 0] = nd.mPos[0] + s % scdim * sc;
     sc_pos[3 * idx + 1] = nd.mPos[1] + (s / scdim) % scdim * sc;
@@ -561,17 +561,23 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
     v->sc_dim = scdim;
     v->sc_per_brick = scpb;
     v->num_sc = num_sc;
-    GV_CUDA(v, v->sc_flag.ensure(sizeof(uint32_t) * (size_t)(nmap + 1), s));
-    GV_CUDA(v, v->sc_map.ensure(sizeof(uint32_t) * (size_t)(nmap + 1), s));
-    GV_CUDA(v, v->sc_cnt.ensure(sizeof(uint32_t) * (size_t)(2 * num_sc + 2), s));
+    GV_CUDA(v, v->sc_cnt.ensure(sizeof(uint32_t) * (size_t)(num_sc + 1), s));
     GV_CUDA(v, v->sc_off.ensure(sizeof(uint32_t) * (size_t)(num_sc + 1), s));
     GV_CUDA(v, v->sc_nid.ensure(sizeof(int32_t) * (size_t)num_sc, s));
     GV_CUDA(v, v->sc_pos.ensure(sizeof(int32_t) * 3 * (size_t)num_sc, s));
-    GV_CUDA(v, cudaMemsetAsync(v->sc_nid.p, 0, sizeof(int32_t) * (size_t)num_sc, s));
-    GV_CUDA(v, cudaMemsetAsync(v->sc_pos.p, 0, sizeof(int32_t) * 3 * (size_t)num_sc, s));
-    k_sc_flag<<<grid_for(nmap, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, v->sc_flag.as<uint32_t>());
-    GV_TRY(exclusive_scan_u32(v, v->sc_flag.as<uint32_t>(), v->sc_map.as<uint32_t>(), nmap));
-    uint32_t *cnt = v->sc_cnt.as<uint32_t>(), *cap = cnt + num_sc + 1;
+    // after a full rebuild every pool leaf is linked: its subcells lie at its pool
+    // index, and every entry of the table is written
+    const uint32_t *mapping = nullptr;
+    if (!v->all_leaves_flagged) {
+        GV_CUDA(v, v->sc_flag.ensure(sizeof(uint32_t) * (size_t)(nmap + 1), s));
+        GV_CUDA(v, v->sc_map.ensure(sizeof(uint32_t) * (size_t)(nmap + 1), s));
+        GV_CUDA(v, cudaMemsetAsync(v->sc_nid.p, 0, sizeof(int32_t) * (size_t)num_sc, s));
+        GV_CUDA(v, cudaMemsetAsync(v->sc_pos.p, 0, sizeof(int32_t) * 3 * (size_t)num_sc, s));
+        k_sc_flag<<<grid_for(nmap, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, v->sc_flag.as<uint32_t>());
+        GV_TRY(exclusive_scan_u32(v, v->sc_flag.as<uint32_t>(), v->sc_map.as<uint32_t>(), nmap));
+        mapping = v->sc_map.as<uint32_t>();
+    }
+    uint32_t *cnt = v->sc_cnt.as<uint32_t>();
     GV_CUDA(v, cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)(num_sc + 1), s));
     ScArgs A;
     A.pos = v->pos;
@@ -585,7 +591,7 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
     A.L = make_lookup(v);
     A.leaves = v->pool_ptr(0);
     A.nleaves = nmap;
-    A.mapping = v->sc_map.as<uint32_t>();
+    A.mapping = mapping;
     A.pmin = make_float3(v->posmin[0], v->posmin[1], v->posmin[2]); // mPosMin, mPosRange (V:5452-5462)
     A.prange = make_float3(v->posmax[0] - v->posmin[0], v->posmax[1] - v->posmin[1], v->posmax[2] - v->posmin[2]);
     A.vmin = make_float3(v->velmin[0], v->velmin[1], v->velmin[2]);
@@ -594,10 +600,7 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
     A.q = A.qvel = nullptr;
     v->sc_fp16 = fp16;
     v->sc_qvel_valid = false;
-    int32_t *status = nullptr;
-    GV_CUDA(v, cudaMallocAsync((void **)&status, sizeof(int32_t), s));
-    GV_CUDA(v, cudaMemsetAsync(status, 0, sizeof(int32_t), s));
-    if (n > 0) k_sc_visit<0><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, nullptr, nullptr, nullptr, status);
+    if (n > 0) k_sc_visit<0><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, nullptr, nullptr);
     GV_TRY(exclusive_scan_u32(v, cnt, v->sc_off.as<uint32_t>(), num_sc));
     uint32_t total = 0;
     GV_CUDA(v, cudaMemcpyAsync(&total, v->sc_off.as<uint32_t>() + num_sc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -605,7 +608,6 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
     v->sc_len = total;
     if (len) *len = (int)total;
     if (total > 0) {
-        GV_CUDA(v, cudaMemcpyAsync(cap, cnt, sizeof(uint32_t) * (size_t)num_sc, cudaMemcpyDeviceToDevice, s));
         GV_CUDA(v, cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)num_sc, s));
         if (fp16) {
             GV_CUDA(v, v->sc_q.ensure(sizeof(uint16_t) * 3 * (size_t)total, s));
@@ -616,20 +618,18 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
                 v->sc_qvel_valid = true;
             }
             if (n > 0)
-                k_sc_visit<2><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, cap, v->sc_off.as<uint32_t>(),
-                                                                         nullptr, status);
+                k_sc_visit<2><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, v->sc_off.as<uint32_t>(), nullptr);
         } else {
             GV_CUDA(v, v->sc_pnt.ensure(sizeof(float) * 3 * (size_t)total, s));
             if (n > 0)
-                k_sc_visit<1><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, cap, v->sc_off.as<uint32_t>(),
-                                                                         v->sc_pnt.as<float>(), status);
+                k_sc_visit<1><<<grid_for(n, 256, 1ll << 31), 256, 0, s>>>(A, cnt, v->sc_off.as<uint32_t>(),
+                                                                         v->sc_pnt.as<float>());
         }
     }
-    k_sc_pos<<<grid_for(nmap * scpb, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, v->sc_map.as<uint32_t>(), sc,
+    k_sc_pos<<<grid_for(nmap * scpb, 256, 1ll << 31), 256, 0, s>>>(v->pool_ptr(0), nmap, mapping, sc,
                                                                    scdim, scpb, num_sc, v->sc_nid.as<int32_t>(),
                                                                    v->sc_pos.as<int32_t>());
     GV_CUDA(v, cudaGetLastError());
-    cudaFreeAsync(status, s);
     return GVDB2_OK;
 }
 

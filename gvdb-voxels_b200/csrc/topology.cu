@@ -50,9 +50,10 @@ inline float ord2f(int32_t o) {
 
 // An empty bounding box.  (A copy of six words from pageable memory holds the
 // host up longer than this launch.)
-__global__ void k_bbox_init(int32_t *bbox) {
-    if (threadIdx.x < 6) bbox[threadIdx.x] = threadIdx.x < 3 ? f2ord(INFINITY) : f2ord(-INFINITY);
+__global__ void k_bbox_init(int32_t *bbox, int32_t lo, int32_t hi) {
+    if (threadIdx.x < 6) bbox[threadIdx.x] = threadIdx.x < 3 ? lo : hi;
 }
+constexpr int32_t kOrdInf = 0x7F800000, kOrdNegInf = (int32_t)0x807FFFFF; // f2ord of the infinities
 
 // GetBoundingBox (V:5404-5467): min/max of pos + trans over all points.
 __global__ void k_bbox(PointsView pos, int64_t n, float3 t, int32_t *bbox) {
@@ -860,7 +861,7 @@ __global__ void k_mark_bits(PointsView pos, int64_t n, float3 orig, float radius
 // word, a lane per bit; of the lanes whose bits share a parent one sets it.
 // Bound by latency, not by the few KB it reads.  A thread per parent that
 // read its up to 512 children's bits one after the other took 28 us on a
-// 27^3-brick grid; a warp per word takes 3 us.
+// 27^3-brick grid; a warp per word takes 4 us.
 __global__ void k_parent_bits(BitGrid C, BitGrid P, int sh) {
     const int nbits = C.d[0] * C.d[1] * C.d[2]; // <= 2^22 (kLargeGridBits)
     const int lane = threadIdx.x & 31;
@@ -1379,7 +1380,7 @@ gvdb2_status rebuild_topology(Volume *v, int n, float radius, const float orig[3
     GV_TRY(ensure_small_words(v));
     reserve_pool(v, n);
     // GetBoundingBox
-    k_bbox_init<<<1, 32, 0, s>>>(dev_words(v)->bbox);
+    k_bbox_init<<<1, 32, 0, s>>>(dev_words(v)->bbox, kOrdInf, kOrdNegInf);
     if (n > 0)
         k_bbox<<<std::min(grid_for(n, 256), 8 * kSmCount), 256, 0, s>>>(v->pos, n, make_float3(orig[0], orig[1], orig[2]),
                                                                         dev_words(v)->bbox);
@@ -1530,8 +1531,7 @@ gvdb2_status compute_bounds(Volume *v) {
     if (n == 0) return GVDB2_OK; // the reference reads leaf 0, which does not exist: bounds unchanged
     cudaStream_t s = v->stream;
     GV_TRY(ensure_small_words(v));
-    const int32_t init[6] = {INT32_MAX, INT32_MAX, INT32_MAX, INT32_MIN, INT32_MIN, INT32_MIN};
-    GV_CUDA(v, cudaMemcpyAsync(dev_words(v)->bbox, init, sizeof(init), cudaMemcpyHostToDevice, s));
+    k_bbox_init<<<1, 32, 0, s>>>(dev_words(v)->bbox, INT32_MAX, INT32_MIN);
     k_leaf_bounds<<<std::min(grid_for(n, 256), 4 * kSmCount), 256, 0, s>>>(v->pool_ptr(0), n, (int)v->range(0),
                                                                            dev_words(v)->bbox);
     GV_CUDA(v, cudaGetLastError());
