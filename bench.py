@@ -550,15 +550,15 @@ def run_ours(a):
 # bricks.  Traffic grows with the brick count at a fixed density, so a
 # launch moves about this many bytes x bricks.
 TRAFFIC_PER_BRICK = {
-    # k_pack_amounts, k_scatter_part, k_scatter_cells, k_scatter_merge
-    "scatter": ((33.6 + 1.0) + (66.8 + 14.0) + (8.9 + 7.4) + (88.4 + 4.6)) * 1e6 / 3240,
+    # k_sort_rows, k_pack_amounts, k_scatter_rows, k_scatter_owner, k_scatter_merge
+    "scatter": ((33.9 + 0.4) + (33.6 + 0.3) + (76.3 + 11.4) + (9.9 + 8.4) + (88.8 + 5.3)) * 1e6 / 3240,
     # k_gather_tile, k_gather_light
-    "gather": ((70.6 + 2.7) + (12.4 + 0.0)) * 1e6 / 3240,
+    "gather": ((71.4 + 3.7) + (12.4 + 0.0)) * 1e6 / 3240,
 }
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 2,097,152-point block at the "
                   "16,777,216-point step's density, scaled by bricks")
-STAGE_KERNELS = {"scatter": "scatter stage: k_pack_amounts<4> + k_scatter_part<cubic,4> (dense cells' partials) + "
-                            "k_scatter_cells<cubic,4> (owner-computes) + k_scatter_merge<cubic,4>",
+STAGE_KERNELS = {"scatter": "scatter stage: k_sort_rows + k_pack_amounts<4> + k_scatter_rows<4> (dense cells' partials) + "
+                            "k_scatter_owner<cubic,4> (owner-computes) + k_scatter_merge<cubic,4>",
                  "gather": "k_gather_tile<cubic,fwd,3> + k_gather_light<cubic,fwd,3>", "apron": "k_apron"}
 
 

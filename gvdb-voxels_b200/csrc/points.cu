@@ -149,11 +149,12 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // ceil(k / slice) work items (cell, slice, slices, accumulator slot) and,
 // when that is more than one, an accumulator slot for its integer sums.
 // With rows_on the dense cells of kRowsMin to kRowsMax points are listed in
-// `rows` instead of the work items.  Cells of at most `light` (<= kLightCell) points are light.  The cells of more
-// than kLightOwn points that are not dense and, for the cubic, those with a face
-// neighbour of more than kHeavyFace (not dense either) are listed in `owner`.  It depends on
-// the cell and its neighbours alone, so that a cloud of a batch gets what a
-// volume of its own gets.
+// `rows` instead of the work items.  Cells of at most `light` (<= kLightCell)
+// points are light.  The cells of more than kLightOwn points that are not dense
+// and, for the cubic, those with a face neighbour of more than kHeavyFace (not
+// dense either) are listed in `owner`.  It depends on the cell and its
+// neighbours alone, so that a cloud of a batch gets what a volume of its own
+// gets.
 // reg_off holds each (cell, region) bin's first entry; off[c] = reg_off[27 c], each
 // cell's (c = ncell: the end), is written for the kernels that follow.
 __global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int2 *tiles,

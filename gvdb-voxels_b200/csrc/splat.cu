@@ -7,13 +7,15 @@
 //   GatherDensity / GatherLevelSet (V:5318-5373, P:696-773): per voxel of
 //     each subcell, max(r - |p - v|) / min(|p - v| - r) over its list.
 // Kernel splats (no reference counterpart): tent (r=1) and cubic B-spline
-// (r=2) scatter onto brick interiors and gather back to points.  One CTA
-// owns one atlas slot: it accumulates the brick interior in shared memory
-// from the brick's own points and the boundary regions of its 26
-// neighbours (binning in points.cu), then writes the interior once with
-// coalesced stores -- no global atomics, no zero-fill pass.  The gather
-// stages the brick plus a 1- or 2-voxel halo from the neighbours'
-// interiors in shared memory and serves all of the brick's points from it.
+// (r=2) scatter onto brick interiors and gather back to points, in cells of
+// 8^3 voxels.  A warp owns a cell: it adds the cell's own points and those of
+// the boundary regions of its 26 neighbours (binning in points.cu) in
+// registers and writes the cell once -- no global atomics, no zero-fill pass;
+// a dense cell's points are summed once into a partial of their own, which a
+// merge adds to the cells that it covers.  The gather stages a cell plus a 1-
+// or 2-voxel halo from the neighbours' interiors in shared memory and serves
+// the cell's points from it, or reads the taps of cells of few points from
+// the atlas.
 #include <algorithm>
 
 #include "dev_common.cuh"
@@ -633,8 +635,9 @@ __device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *
 // them zero (4 of the 8 rows): bound by instruction issue and by the latency
 // of the records' reads (43% of issue slots with 14 warps an SM; shared memory
 // for 20 KB a cell bounds them: with a fifth plane, which spares a barrier a
-// plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points).  The fixed-point atomics of k_scatter_part, two per tap and
-// channel, are bound by the shared-memory atomic rate, 30 of 32 lanes a cycle.
+// plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points).  The fixed-point atomics
+// of k_scatter_part, two per tap and channel, are bound by the shared-memory
+// atomic rate, 30 of 32 lanes a cycle.
 //
 // Sums are float, at most some 20 terms in a register window, then up to 8
 // such sums per voxel.
@@ -1359,9 +1362,6 @@ __device__ __forceinline__ void sc_sort_chunk(ScChunk &C, int fill, int lane) {
 
 #ifndef GVDB2_SC_PIPE
 #define GVDB2_SC_PIPE 0
-#endif
-#ifndef GVDB2_SC_PREFETCH
-#define GVDB2_SC_PREFETCH 0
 #endif
 // A record's values that lane (y, q) reads.
 struct ScRec {
