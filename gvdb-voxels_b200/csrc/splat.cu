@@ -2159,8 +2159,9 @@ __device__ __forceinline__ void gather_light_point(const GatherArgs &G, int64_t 
         const int ex = step(lx + N - 1), ey = step(ly + N - 1), ez = step(lz + N - 1);
         const int cutx = ex == sx ? N : (ex == 0 ? -lx : res - lx), cuty = ey == sy ? N : (ey == 0 ? -ly : res - ly),
                   cutz = ez == sz ? N : (ez == 0 ? -lz : res - lz);
-        // element offset of the stencil's first tap in each of the up to 8 bricks;
-        // where there is none, one that stays below 0 for every tap
+        // element offset of the stencil's first tap in each of the up to 8 bricks (with no
+        // apron, below 0 in the upper bricks of slot 0's first rows, whose own taps are
+        // not); where there is no brick, one that stays below 0 for every tap
         constexpr int64_t none = -(int64_t(1) << 40);
         int64_t at[2][2][2];
 #pragma unroll
@@ -2182,9 +2183,9 @@ __device__ __forceinline__ void gather_light_point(const GatherArgs &G, int64_t 
             const int64_t o1 = (bz ? (by ? at[1][1][1] : at[1][0][1]) : (by ? at[0][1][1] : at[0][0][1])) + r;
 #pragma unroll
             for (int tx = 0; tx < N; tx++) {
-                const int64_t o = tx >= cutx ? o1 : o0;
+                const int64_t o = (tx >= cutx ? o1 : o0) + tx;
 #pragma unroll
-                for (int c = 0; c < NCH; c++) g[tx][c] = o >= 0 ? __ldg(G.chan[c] + o + tx) : 0.0f;
+                for (int c = 0; c < NCH; c++) g[tx][c] = o >= 0 ? __ldg(G.chan[c] + o) : 0.0f;
             }
         };
     };
