@@ -635,12 +635,25 @@ __device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *
 // them zero (4 of the 8 rows): bound by instruction issue and by the latency
 // of the records' reads (43% of issue slots with 14 warps an SM; shared memory
 // for 20 KB a cell bounds them: with a fifth plane, which spares a barrier a
-// plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points).  The fixed-point atomics
+// plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points, one window).  The
+// loop over first columns is not unrolled: its 9 copies cost 0.4 ms more.  The fixed-point atomics
 // of k_scatter_part, two per tap and channel, are bound by the shared-memory
 // atomic rate, 30 of 32 lanes a cycle.
 //
-// Sums are float, at most some 20 terms in a register window, then up to 8
-// such sums per voxel.
+// Sums are float, in two windows that take every other point.  However the
+// points lie, a register takes at most kRowFold / 2 terms a first column, 4 of
+// which a column's stay spans, before the windows are folded into the planes: a
+// sum of two floats whose remainder stays in the window.  A partial is so as
+// close to 64 bits as the fixed-point one (float weights and products, exact
+// sums).  Largest error over the largest value, mean of 40 cells in a float32
+// restatement, fixed point / so / one window without folds: 768 points spread
+// evenly 1.35e-7 / 1.15e-7 / 1.39e-7, 2,048 of them 1.29e-7 / 1.10e-7 / 2.04e-7;
+// a lattice of 1,024 1.59e-7 / 1.57e-7 / 2.17e-7; 1,200 points in one voxel
+// 0.95e-7 / 0.33e-7 / 2.16e-7; 1,200 equal points of equal amounts 1.19e-7 /
+// 0.90e-7 / 89e-7.  First columns of many points, whose partial sums of amounts of
+// both signs outgrow the result, are folded more often.  The second window and the
+// folds cost 28 us of 1.18 ms for 16.7M lattice points.
+constexpr uint32_t kRowFold = 12, kRowMany = 32, kRowFoldMany = 4;
 constexpr int kRowKeys = 2 * 9 * 9; // (half, z0, x0)
 constexpr int kRowOff = kRowKeys + 2;
 constexpr int kSortThreads = 192, kSortWarps = kSortThreads / 32;
@@ -842,22 +855,13 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
                 int t = turn + tz;
                 if (t >= 4) t -= 4;
                 V *row = M.plane[half][t][ty];
-                float2 acc[4][NP];
+                // two windows, columns x0 to x0 + 3, which take the points of a pair
+                float2 acc[2][4][NP];
 #pragma unroll
                 for (int k = 0; k < 4; k++)
 #pragma unroll
-                    for (int c = 0; c < NP; c++) acc[k][c] = make_float2(0.0f, 0.0f);
-                auto flush = [&](int x, int k) { // window column k (x modulo 4) to column x of the planes
-                    float g[4] = {0.f, 0.f, 0.f, 0.f};
-                    gvec_get<NCH>(row[x], g);
-                    float sum[NCH];
-#pragma unroll
-                    for (int c = 0; c < NCH; c++) sum[c] = g[c] + ((c & 1) ? acc[k][c / 2].y : acc[k][c / 2].x);
-                    gvec_put<NCH>(row[x], sum);
-#pragma unroll
-                    for (int c = 0; c < NP; c++) acc[k][c] = make_float2(0.0f, 0.0f);
-                };
-                auto add = [&](const Rec &p, int x0) {
+                    for (int c = 0; c < NP; c++) acc[0][k][c] = acc[1][k][c] = make_float2(0.0f, 0.0f);
+                auto add = [&](const Rec &p, float2 (&win)[4][NP]) {
                     const float2 ap[2] = {make_float2(p.a.x, p.a.y), make_float2(p.a.z, p.a.w)};
                     const float2 w[4] = {make_float2(p.x01.x, p.x01.y), make_float2(p.x01.z, p.x01.w),
                                          make_float2(p.x23.x, p.x23.y), make_float2(p.x23.z, p.x23.w)};
@@ -865,35 +869,83 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
                     for (int c = 0; c < NP; c++) {
                         const float2 t2 = __fmul2_rn(ap[c], make_float2(p.wyz, p.wyz));
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            acc[(x0 + k) & 3][c] = __ffma2_rn(t2, w[k], acc[(x0 + k) & 3][c]);
+                        for (int k = 0; k < 4; k++) win[k][c] = __ffma2_rn(t2, w[k], win[k][c]);
                     }
                 };
+                auto join = [&](int k) { // both windows' sums of a column, in the first one
 #pragma unroll
+                    for (int c = 0; c < NP; c++) {
+                        acc[0][k][c] = __fadd2_rn(acc[0][k][c], acc[1][k][c]);
+                        acc[1][k][c] = make_float2(0.0f, 0.0f);
+                    }
+                };
+                auto sum_of = [&](int k, int c) -> float & { return (c & 1) ? acc[0][k][c / 2].y : acc[0][k][c / 2].x; };
+                auto flush = [&](int x, int k) { // the windows' column k to column x of the planes
+                    join(k);
+                    float g[4] = {0.f, 0.f, 0.f, 0.f}, sum[NCH];
+                    gvec_get<NCH>(row[x], g);
+#pragma unroll
+                    for (int c = 0; c < NCH; c++) sum[c] = g[c] + sum_of(k, c);
+                    gvec_put<NCH>(row[x], sum);
+                };
+#pragma unroll 1
                 for (int x0 = 0; x0 < 9; x0++) {
                     const uint32_t e = off[x0 + 1];
+                    // points of this first column until the windows are folded
+                    const uint32_t step = e - i > kRowMany ? kRowFoldMany : kRowFold;
+                    uint32_t full = i + step;
                     while (i < e) {
                         if (i == staged) {
                             stage(i);
                             staged = i + 32;
                         }
-                        const uint32_t m = min(e, staged);
+                        if (i == full) {
+                            // to the planes, what the rounding of each sum leaves out staying
+                            // in the first window
+                            full += step;
+                            float g[4][4];
+#pragma unroll
+                            for (int k = 0; k < 4; k++) gvec_get<NCH>(row[x0 + k], g[k]);
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                float sum[NCH];
+                                join(k);
+#pragma unroll
+                                for (int c = 0; c < NCH; c++) {
+                                    float &a = sum_of(k, c);
+                                    sum[c] = g[k][c] + a;
+                                    const float d = sum[c] - g[k][c];
+                                    a = (g[k][c] - (sum[c] - d)) + (a - d);
+                                }
+                                gvec_put<NCH>(row[x0 + k], sum);
+                            }
+                        }
+                        const uint32_t m = min(min(e, staged), full);
                         const float *r = M.rec[half][32 + i - staged];
                         for (; i + 1 < m; i += 2, r += 2 * kRowRec) { // two at a time: their reads overlap
                             const Rec p = load(r), q = load(r + kRowRec);
-                            add(p, x0);
-                            add(q, x0);
+                            add(p, acc[0]);
+                            add(q, acc[1]);
                         }
                         if (i < m) {
-                            add(load(r), x0);
+                            add(load(r), acc[0]);
                             i++;
                         }
                     }
-                    // no later point reaches column x0
-                    if (e > off[x0 > 3 ? x0 - 3 : 0]) flush(x0, x0 & 3);
+                    if (e > off[x0 > 3 ? x0 - 3 : 0]) { // else the windows are empty
+                        flush(x0, 0); // no later point reaches column x0
+#pragma unroll
+                        for (int c = 0; c < NP; c++)
+#pragma unroll
+                            for (int w = 0; w < 2; w++) {
+#pragma unroll
+                                for (int k = 0; k < 3; k++) acc[w][k][c] = acc[w][k + 1][c];
+                                acc[w][3][c] = make_float2(0.0f, 0.0f);
+                            }
+                    }
                 }
 #pragma unroll
-                for (int x = 9; x < X::E; x++) flush(x, x & 3);
+                for (int k = 0; k < 3; k++) flush(9 + k, k);
             }
         }
         __syncthreads(); // both halves are done with plane z0

@@ -1,0 +1,53 @@
+"""GPU parity of the cubic splat's cells of 768 to 2,048 points, whose sums are taken in float registers, where those sums
+can go wrong: however many of a cell's points share a stencil."""
+import numpy as np
+import pytest
+
+from _helpers import interior, make_oracle
+from test_gpu_topology import gpu_volume
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -24
+# Roundings on the way to a voxel, each at most U of the sum of the |contributions|: three weights of at most 4 each, two
+# products, 32 terms of a window column (8 a first column, 4 of them), 8 sums in a plane's column, 8 partials merged
+ROWS_TOL = (3 * 4 + 2 + 32 + 8 + 8) * U
+
+
+def cell_points(kind, n, rng):
+    """n points in the cell [80, 88)^3."""
+    if kind == "uniform":
+        return rng.uniform(80.0, 87.99, (n, 3))
+    if kind == "voxel":
+        return rng.uniform(83.51, 84.49, (n, 3))
+    if kind == "coincident":
+        return np.tile((84.7, 83.3, 83.9), (n, 1))
+    q = rng.uniform(80.0, 87.99, (n, 3))
+    q[:, 1:] = (83.3, 84.9)
+    return q  # a line along x
+
+
+@pytest.mark.parametrize("amounts", ["equal", "positive", "signed"])
+@pytest.mark.parametrize("kind", ["uniform", "voxel", "coincident", "line"])
+@pytest.mark.parametrize("n", [768, 1031, 2048])
+@pytest.mark.parametrize("nch", [1, 4])
+def test_sums_of_points_that_share_a_stencil(gvdb2_mod, oracle_mod, amounts, kind, n, nch):
+    import torch
+    rng = np.random.default_rng(32)
+    pts = np.concatenate([cell_points(kind, n, rng), [[100.0, 100.0, 100.0]]]).astype(np.float32)
+    a = {"equal": np.full((n + 1, nch), 1.1), "positive": rng.uniform(0.5, 1.5, (n + 1, nch)),
+         "signed": rng.normal(size=(n + 1, nch))}[amounts].astype(np.float32)
+    chans, grads = list(range(nch)), list(range(nch, 2 * nch))
+    o = make_oracle(oracle_mod, chans=chans + grads)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.update_atlas()
+    v = gpu_volume(gvdb2_mod, pts, chans=chans)
+    v.RebuildTopology(len(pts), 2.0)
+    v.UpdateAtlas()
+    ta = torch.from_numpy(a).cuda()
+    v.ScatterKernel(2, len(pts), chans, attrs=[(ta, c) for c in chans])
+    o.scatter_kernel(2, pts, chans, attrs=[a[:, c] for c in chans])
+    o.scatter_kernel(2, pts, grads, attrs=[np.abs(a[:, c]) for c in chans])
+    for c in chans:
+        err = np.abs(interior(v.atlas(c), 1).astype(np.float64) - interior(o.atlas(c), 1)).max()
+        assert err <= ROWS_TOL * interior(o.atlas(grads[c]), 1).max()
