@@ -218,7 +218,7 @@ constexpr uint32_t kSlicePts = 4096;
 constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntOwner = 6,
               kCntRows = 7, kCntTiles = 8, kCntWords = 12;
 // Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic): 16.7M
-// points in cells of 1,024 on average, 4 channels, 1.18 + 0.13 ms (its sort)
+// points in cells of 1,024 on average, 4 channels, 1.18 + 0.15 ms (its sort)
 // against 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162
 // short units (a 300,000-point blob's cells of 512 to 700: 48 us against 20), more
 // make a cell its launch's tail.
