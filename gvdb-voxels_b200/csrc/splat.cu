@@ -754,6 +754,10 @@ struct PartPos {
 };
 __device__ constexpr PartPos kPartPos{};
 
+__device__ __forceinline__ bool all_finite(float4 a) {
+    return isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w);
+}
+
 constexpr int kRowRec = 24; // floats a record: x weights twice each, 8 y weights, z weights, amounts
 template <int NCH>
 struct RowSmem {
@@ -762,6 +766,7 @@ struct RowSmem {
     typename GVec<NCH>::T plane[2][4][8][13];
     float rec[2][32][kRowRec];
     uint16_t off[kRowOff];
+    uint16_t special; // some point's amounts are not all finite
 };
 
 template <int NCH>
@@ -789,6 +794,7 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
     const int ox = nd.mPos[0] + kCell * cx - X::H, oy = nd.mPos[1] + kCell * cy - X::H,
               oz = nd.mPos[2] + kCell * cz - X::H;
     for (int i = threadIdx.x; i <= kRowKeys; i += 64) M.off[i] = row_off[(int64_t)pslot * kRowOff + i];
+    if (threadIdx.x == 0) M.special = 0;
     {
         float *z = reinterpret_cast<float *>(M.plane);
         for (int i = threadIdx.x; i < (int)(sizeof(M.plane) / sizeof(float)); i += 64) z[i] = 0.0f;
@@ -813,8 +819,13 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
         }
     };
     auto stage = [&](uint32_t i0) { // records of points [i0, i0 + 32), fetched before
-        const float4 q = next_q, am = next_am;
+        const float4 q = next_q;
+        float4 am = next_am;
         fetch(i0 + 32);
+        if (!all_finite(am)) { // times the zero weights it would reach rows beyond its stencil
+            am = make_float4(0.f, 0.f, 0.f, 0.f);
+            M.special = 1;
+        }
         float *r = M.rec[half][lane];
         float4 *r4 = reinterpret_cast<float4 *>(r);
         const int32_t cloud = __float_as_int(q.w);
@@ -973,6 +984,35 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
         }
         turn = turn == 3 ? 0 : turn + 1;
         __syncthreads(); // the next units add to this plane's place
+    }
+    // The points left out, in sorted order, by one warp: two taps a lane, added to
+    // the partial in memory, which the CTA has written.
+    if (!M.special || half != 0) return;
+    for (uint32_t i0 = 0; i0 < R; i0 += 32) {
+        int32_t j = i0 + lane < R ? order[beg + i0 + lane] : -1;
+        if (j >= 0 && !in_range(S.lim, j, S.lim.nentry, 43)) j = -1;
+        unsigned left = __ballot_sync(0xffffffffu, j >= 0 && !all_finite(S.bin_amt[max(j, 0)]));
+        for (; left; left &= left - 1) {
+            const int32_t p = __shfl_sync(0xffffffffu, j, __ffs(left) - 1);
+            const float4 q = S.bin_pos[p], am = S.bin_amt[p];
+            const float a4[4] = {am.x, am.y, am.z, am.w};
+            const int32_t cloud = __float_as_int(q.w);
+            int3 o = make_int3(0, 0, 0);
+            if (cloud >= 0 && in_range(S.lim, cloud, S.lim.ncloud, 44))
+                o = make_int3(S.pos.origin[3 * cloud], S.pos.origin[3 * cloud + 1], S.pos.origin[3 * cloud + 2]);
+            float wx[4], wy[4], wz[4];
+            const int fx = T::eval_fine(q.x, wx) + o.x - ox, fy = T::eval_fine(q.y, wy) + o.y - oy,
+                      fz = T::eval_fine(q.z, wz) + o.z - oz;
+            if ((unsigned)fx > 8u || (unsigned)fy > 8u || (unsigned)fz > 8u) continue;
+            for (int t = lane; t < 64; t += 32) {
+                const int tx = t & 3, ty = (t >> 2) & 3, tz = t >> 4;
+                const float w = wx[tx] * wy[ty] * wz[tz];
+                const int pos = kPartPos.pos[((fz + tz) * X::E + fy + ty) * X::E + fx + tx];
+#pragma unroll
+                for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] += a4[c] * w;
+            }
+            __syncwarp(); // the next point may reach the same voxels
+        }
     }
 }
 

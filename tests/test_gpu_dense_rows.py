@@ -71,3 +71,33 @@ def test_bit_reproducible_whatever_the_binning(gvdb2_mod):
         want = want or got
         for g, w in zip(got, want):
             assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("nch", [1, 3])
+@pytest.mark.parametrize("n", [768, 2048])
+def test_amounts_that_are_not_finite(gvdb2_mod, oracle_mod, nch, n):
+    """Infinite and NaN amounts reach the voxels of their own stencils and no others; the rest of the cell and the
+    channels whose amounts are finite are those of the FP64 oracle, to the bound above."""
+    import torch
+    rng = np.random.default_rng(34)
+    pts = np.concatenate([rng.uniform(80.0, 87.99, (n, 3)), [[100.0, 100.0, 100.0]]]).astype(np.float32)
+    pts[:4] = [[81.3, 81.4, 81.2], [86.8, 81.7, 86.6], [81.7, 86.7, 82.4], [81.9, 86.2, 82.3]]
+    a = rng.uniform(0.5, 1.5, (n + 1, nch)).astype(np.float32)
+    a[:4, nch - 1] = (np.inf, np.nan, -np.inf, np.inf)
+    chans = list(range(nch))
+    o = make_oracle(oracle_mod, chans=chans)
+    assert o.rebuild_topology(pts, 2.0) == 0
+    o.update_atlas()
+    v = gpu_volume(gvdb2_mod, pts, chans=chans)
+    v.RebuildTopology(len(pts), 2.0)
+    v.UpdateAtlas()
+    ta = torch.from_numpy(a).cuda()
+    v.ScatterKernel(2, len(pts), chans, attrs=[(ta, c) for c in chans])
+    o.scatter_kernel(2, pts, chans, attrs=[a[:, c] for c in chans])
+    for c in chans:
+        g, w = interior(v.atlas(c), 1).astype(np.float64), interior(o.atlas(c), 1)
+        assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(np.isinf(g), np.isinf(w))
+        ok = np.isfinite(w)
+        assert np.array_equal(g[np.isinf(w)], w[np.isinf(w)])
+        assert np.abs(g[ok] - w[ok]).max() <= ROWS_TOL * np.abs(w[ok]).max()
+    assert np.isnan(w).any() and np.isinf(w).any()
