@@ -213,10 +213,11 @@ __device__ __forceinline__ bool in_range(const SplatLimits &L, int64_t i, int64_
 }
 constexpr uint32_t kSlicePts = 4096;
 // cell_cnt entries: huge, heavy, light cells; dense cells, dense work
-// items (slices), dense cells of more than one slice, cells listed for
-// k_scatter_cells, dense cells listed for k_scatter_rows, items of huge cells
-constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntOwner = 6,
-              kCntRows = 7, kCntTiles = 8, kCntWords = 12;
+// items (slices), dense cells of more than one slice, dense cells listed for
+// k_scatter_rows, items of huge cells,
+// cells of each class of sources
+constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntRows = 6,
+              kCntTiles = 7, kCntSrc = 8, kCntWords = 14;
 // Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic): 16.7M
 // points in cells of 1,024 on average, 4 channels, 1.18 + 0.15 ms (its sort)
 // against 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162
@@ -230,20 +231,37 @@ constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWor
 #endif
 constexpr int kRowsMin = GVDB2_ROWS_MIN, kRowsMax = GVDB2_ROWS_MAX;
 static_assert(kRowsMax <= 65535, "16-bit positions in a cell");
-// Most points of a cell that k_scatter_light serves, and (cubic) of its face
-// neighbours, dense cells not counted.  Scatter passes at 32, 64 and 96 points:
-// one channel, 612k cells of 9 points on average 1.49, 1.42, 1.39 ms; three
-// channels, a 300,000-point blob 146, 141, 138 us; four channels, 634k cells of 26
-// points 4.98, 4.86, 4.78 ms.  Without the rule on neighbours the cells around a
-// block of 256 points a cell (four channels) cost 35 us of 795; with it 18 us.
-#ifndef GVDB2_LIGHT_OWN
-#define GVDB2_LIGHT_OWN 96
-#endif
-#ifndef GVDB2_HEAVY_FACE
-#define GVDB2_HEAVY_FACE 192
-#endif
-constexpr int32_t kPartListed = -2; // a cell's partial slot when it is listed for k_scatter_cells
-constexpr int kLightOwn = GVDB2_LIGHT_OWN, kHeavyFace = GVDB2_HEAVY_FACE;
+// A cell has an estimate of the points that reach it, dense cells' left out: its own
+// and, for the cubic (whose stencils reach 1.5 voxels past a face, of 8), 3/16 of
+// its face neighbours'.  The owner-computes pass takes the cells class by class, class
+// k having more than edge[k] and no more than edge[k - 1] (the last, the rest).
+constexpr int kSrcClasses = 6;
+static_assert(kCntSrc + kSrcClasses == kCntWords, "a count per class");
+struct SrcEdges {
+    int edge[kSrcClasses - 1];
+};
+// The first classes take k_scatter_cells, the others k_scatter_light, by kernel and
+// channels.  Measured on even clouds of 2, 6, 12, ... 140 points a cell (2M and 8M
+// points), all cells in the one and all in the other: the light form is the faster
+// up to 128, 128, 48 and 32 (tent, 1 to 4 channels) and 200, 72, 24 and 24 (cubic),
+// at 12 points a cell 0.51, 0.67, 0.85, 0.92 and 0.60, 0.73, 1.01, 1.00 of the
+// other's time, at 50 cubic points 0.89, 1.05, 1.27, 1.31.
+constexpr SrcEdges kSrcEdges[2] = {{254, 128, 64, 48, 32}, {254, 200, 120, 72, 24}};
+constexpr int kOwnerClasses[2][4] = {{2, 2, 4, 5}, {2, 4, 5, 5}};
+// Where half of the cells or more are of the last class, most of them without a
+// point, the light form waits for the writes of zeros and takes the cells of some
+// points along: a scene of 634,000 32^3-brick cells, 16.8M points, 4 channels 4.84 ms
+// with 2 classes in k_scatter_cells, 5.24 with 5.
+constexpr int kOwnerClassesSparse = 2;
+// The same in k_scatter_owner, whose registers and shared memory the light form, the
+// last class, then has to live with: 300,000 points, tent 0.89 at 6 points a cell, 1.01
+// at 25 and 1.11 at 70, cubic 0.49 to 0.91 at 2, 0.97 to 1.05 at 6, 1.12 at 12.
+constexpr SrcEdges kSrcEdgesOne[2] = {{254, 128, 64, 32, 18}, {254, 128, 64, 24, 8}};
+// Up to two and a half times the cells that run at a time, of few points each, there
+// is no order to gain from: 4,973 cells of 4 points 15 us in either, and the list
+// takes 4 (5,653 cells of 177 points 86 us in cell order, 60 in the list's).
+constexpr int64_t kOrderCells = kSmCount * 16 * 5 / 2, kOrderPoints = 8;
+constexpr int kListCells = 256; // cells per block of k_cell_list and k_owner_list
 // cell of a voxel inside its brick (local voxel coordinates in [0, res0))
 __device__ __forceinline__ int cell_of_local(int lx, int ly, int lz, int m) {
     return ((lz >> 3) * m + (ly >> 3)) * m + (lx >> 3);

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <array>
 #include <functional>
 #include <string>
 #include <vector>
@@ -201,8 +202,14 @@ struct Volume {
     // cells whose voxels k_scatter_merge adds partials to (count in the
     // last 16 bytes)
     DevBuf merge_list;
-    // cells of more than kLightOwn points that are not dense
-    DevBuf cell_owner;
+    // the cells in the order that the owner-computes pass takes them, class by
+    // class of sources; how many of the first take k_scatter_cells for 1 to 4
+    // channels (-1: not read back), and which classes; the cells' classes, their counts per block of cells, and
+    // the cells of k_scatter_light in cell order
+    DevBuf cell_owner, cell_cls, cell_blk, light_list;
+    bool ordered = false; // cell_owner is made
+    std::array<int64_t, 4> src_cells{-1, -1, -1, -1};
+    std::array<int, 4> src_classes{};
     int64_t dense_cap = 0, work_cap = 0, multi_cap = 0, part_acc_cap = 0;
     // the dense cells that k_scatter_rows takes (cubic): their list and its
     // capacity, their keys' first positions (the sorted order itself is in
@@ -337,6 +344,8 @@ int32_t *splat_guard_word(Volume *v);
 
 // ---- points.cu ----
 gvdb2_status insert_points(Volume *v, int n, const float trans[3], int prefix);
+// makes light_list from the bins of a volume of many cells
+gvdb2_status light_list(Volume *v, int64_t ncell, int first);
 gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]);
 gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const float trans[3], int *len,
                                    bool fp16 = false);

@@ -237,11 +237,15 @@ struct SplatArgs {
     float *part;
     int32_t *part_acc;
     uint32_t *part_done;
-    // cells with a dense cell among their 27 (k_scatter_cells lists them)
+    // cells with a dense cell among their 27, listed by the owner-computes pass
     int32_t *merge_list;
     uint32_t *merge_cnt;
-    // the cells of k_scatter_cells: more than kLightOwn points, not dense
-    const int32_t *owner_list;
+    // the cells in order of the owner-computes pass (nullptr: in cell order), their
+    // classes of sources, and how many of the first take k_scatter_cells (-1: the
+    // host does not know; all but the last class)
+    const uint8_t *cell_cls;
+    const int32_t *owner_list, *light_list;
+    int64_t owners;
 };
 
 
@@ -1028,8 +1032,8 @@ __device__ __forceinline__ int sc_key(int fx, int fz) {
 
 // ---- owner-computes scatter, cells with few sources ----------------------
 //
-// The same sums as k_scatter_cells below for the cells of at most kLightOwn
-// points (and the dense ones, for their neighbours' points): in sparse volumes
+// The same sums as k_scatter_cells below for the cells that few points reach
+// (SrcEdges; and the dense ones, for their neighbours' points): in sparse volumes
 // most of them, where that kernel's 128 registers and its walks over short runs
 // cost far more than the points do.  One warp per cell adds the sources one after
 // the other, in that kernel's order, to a tile of the cell in shared memory, a
@@ -1107,7 +1111,6 @@ __device__ __forceinline__ void scatter_light_cell(const SplatArgs &S, LightWarp
     using T = Taps<KERNEL>;
     using V = typename GVec<NCH>::T;
     constexpr int N = T::N;
-    if (S.cell_part[cell] == kPartListed) return; // k_scatter_cells's
     int64_t slot;
     int cx, cy, cz;
     cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
@@ -1346,8 +1349,10 @@ template <int KERNEL, int NCH>
 __global__ void __launch_bounds__(32 * kLightWarps) k_scatter_light(SplatArgs S) {
     extern __shared__ __align__(16) unsigned char light_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t cell = (int64_t)blockIdx.x * kLightWarps + warp;
-    if (cell < S.ncell)
+    const int64_t i = (int64_t)blockIdx.x * kLightWarps + warp;
+    if (i >= S.ncell - S.owners) return;
+    const int64_t cell = S.light_list[i];
+    if (in_range(S.lim, cell, S.ncell, 45))
         scatter_light_cell<KERNEL, NCH>(S, reinterpret_cast<LightWarp<NCH> *>(light_smem)[warp], cell, lane);
 }
 
@@ -1795,49 +1800,45 @@ __device__ __forceinline__ void scatter_cell(const SplatArgs &S, ScChunk &C, int
     }
 }
 
-// kScWarps cells per CTA at a time, a warp per cell, of the cells of more than
-// kLightOwn points (SplatArgs::owner_list).  Their number is known on the device
-// only: each warp takes every (blocks * kScWarps)-th cell.
-template <int KERNEL, int NCH>
-__device__ __forceinline__ void scatter_listed_cells(const SplatArgs &S, ScChunk &C, int64_t block, int64_t blocks,
-                                                     int lane, int warp) {
-    const int64_t count = S.cell_cnt[kCntOwner];
-    for (int64_t i = block * kScWarps + warp; i < count; i += blocks * kScWarps) {
-        const int64_t cell = S.owner_list[i];
-        if (!in_range(S.lim, cell, S.ncell, 28)) continue;
-        scatter_cell<KERNEL, NCH>(S, C, cell, lane);
-        __syncwarp(); // the next cell reuses the chunk
-    }
-}
+// kScWarps listed cells per CTA, a warp per cell.
 template <int KERNEL, int NCH>
 __global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_cells(SplatArgs S) {
     extern __shared__ __align__(16) unsigned char sc_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    scatter_listed_cells<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], blockIdx.x, gridDim.x, lane, warp);
+    const int64_t i = (int64_t)blockIdx.x * kScWarps + warp;
+    if (i >= S.owners) return;
+    const int64_t cell = S.owner_list[i];
+    if (!in_range(S.lim, cell, S.ncell, 28)) return;
+    scatter_cell<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], cell, lane);
 }
 
-// Both in one launch, k_scatter_cells's cells in the first `heavy` blocks: in
-// volumes of few cells the longest of these (a warp each) would otherwise run
-// alone.  The same sums, so the host may choose by size.
-template <int KERNEL, int NCH>
-constexpr size_t owner_smem_bytes() {
-    return std::max(sizeof(ScChunk) * kScWarps, sizeof(LightWarp<NCH>) * kLightWarps);
+// Both forms in one launch, for volumes of few cells, in the list's order: the longest
+// cells first.  A warp's shared memory serves either form, so the warps' shares start
+// apart by the larger of the two.  Bound, as k_scatter_cells, by instruction issue:
+// 18,744 cells of 256 points, 4 channels 761 us (with the cells listed in the order
+// of 32-cell atomics and a warp for each listed cell that only left 784).
+template <int NCH>
+constexpr size_t owner_warp_bytes() {
+    return std::max(sizeof(ScChunk), sizeof(LightWarp<NCH>));
 }
 template <int KERNEL, int NCH>
-__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_owner(SplatArgs S, unsigned heavy) {
-    static_assert(kScWarps == kLightWarps, "one block size");
+__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_owner(SplatArgs S) {
+    constexpr size_t share = owner_warp_bytes<NCH>();
+    static_assert(share % 16 == 0, "16-byte accesses");
     extern __shared__ __align__(16) unsigned char sc_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (blockIdx.x < heavy) {
-        scatter_listed_cells<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], blockIdx.x, heavy, lane, warp);
-        return;
-    }
-    const int64_t cell = (int64_t)(blockIdx.x - heavy) * kLightWarps + warp;
-    if (cell < S.ncell)
-        scatter_light_cell<KERNEL, NCH>(S, reinterpret_cast<LightWarp<NCH> *>(sc_smem)[warp], cell, lane);
+    const int64_t i = (int64_t)blockIdx.x * kScWarps + warp;
+    if (i >= S.ncell) return;
+    const int64_t cell = S.owner_list ? (int64_t)S.owner_list[i] : i;
+    if (!in_range(S.lim, cell, S.ncell, 46)) return;
+    unsigned char *mine = sc_smem + warp * share;
+    if (S.cell_cls[cell] < kSrcClasses - 1)
+        scatter_cell<KERNEL, NCH>(S, *reinterpret_cast<ScChunk *>(mine), cell, lane);
+    else
+        scatter_light_cell<KERNEL, NCH>(S, *reinterpret_cast<LightWarp<NCH> *>(mine), cell, lane);
 }
 
-// Adds the dense cells' partials to the cells listed by k_scatter_cells
+// Adds the dense cells' partials to the cells listed by the owner-computes pass
 // (those with a dense cell among their 27): a CTA per listed cell (CTAs
 // past the list's end return), a thread per interior voxel, which adds, in
 // the order of kMergeMap, the partials that cover the voxel to the sum the
@@ -2447,11 +2448,6 @@ gvdb2_status ensure_zeroed(Volume *v, DevBuf &b, size_t bytes) {
     return GVDB2_OK;
 }
 
-// Up to this many cells the owner-computes pass is one launch (k_scatter_owner):
-// above it the light cells, most of such a volume, gain more from the
-// occupancy of a kernel of their own.
-constexpr int64_t kOneLaunchCells = 1 << 16;
-
 // Scatter of up to 4 channels (one group): the channel amounts in bin order,
 // the dense cells' partial sums (a CTA per slice), then the owner-computes
 // pass over every cell of the active bricks (cells no stencil reaches get
@@ -2477,7 +2473,9 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     // the list's count sits in its last 16 bytes
     S.merge_cnt = reinterpret_cast<uint32_t *>(v->merge_list.as<char>() + v->merge_list.bytes - 16);
     S.merge_list = v->merge_list.as<int32_t>();
-    S.owner_list = v->cell_owner.as<int32_t>();
+    S.owner_list = v->ordered ? v->cell_owner.as<int32_t>() : nullptr;
+    S.cell_cls = v->cell_cls.as<uint8_t>();
+    S.owners = v->src_cells[NCH - 1];
     if (v->bin_key.n == 0) GV_CUDA(v, cudaMemsetAsync(S.merge_cnt, 0, sizeof(uint32_t), v->stream));
     if (v->bin_key.n > 0)
         k_pack_amounts<NCH><<<grid_for(v->bin_key.n, 256, 1ll << 31), 256, 0, v->stream>>>(S);
@@ -2496,22 +2494,25 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
         kp<<<(unsigned)v->work_cap, kPartThreads, ps, v->stream>>>(S);
     }
     if (S.ncell > 0) {
-        // blocks for the cells of more than kLightOwn points: a warp each, but no more than 16 rounds
-        const int64_t heavy = std::min<int64_t>({S.ncell, v->bin_key.n / (kLightOwn + 1), (int64_t)64 * kSmCount * kScWarps});
-        const unsigned hb = (unsigned)((heavy + kScWarps - 1) / kScWarps);
-        const unsigned lb = (unsigned)((S.ncell + kLightWarps - 1) / kLightWarps);
-        if (S.ncell <= kOneLaunchCells) {
-            constexpr size_t os = owner_smem_bytes<KERNEL, NCH>();
+        const int64_t past = S.owners;
+        if (past < 0) { // few cells, listed with the bins
+            constexpr size_t os = owner_warp_bytes<NCH>() * kScWarps;
             auto ko = k_scatter_owner<KERNEL, NCH>;
             GV_TRY(launch_smem(v, ko, os, "scatter"));
-            ko<<<hb + lb, 32 * kScWarps, os, v->stream>>>(S, hb);
+            ko<<<(unsigned)((S.ncell + kScWarps - 1) / kScWarps), 32 * kScWarps, os, v->stream>>>(S);
         } else {
-            constexpr size_t ls = sizeof(LightWarp<NCH>) * kLightWarps;
-            auto kl = k_scatter_light<KERNEL, NCH>;
-            GV_TRY(launch_smem(v, kl, ls, "scatter"));
-            GV_TRY(launch_smem(v, k, smem, "scatter"));
-            if (hb > 0) k<<<hb, 32 * kScWarps, smem, v->stream>>>(S);
-            kl<<<lb, 32 * kLightWarps, ls, v->stream>>>(S);
+            if (past > 0) {
+                GV_TRY(launch_smem(v, k, smem, "scatter"));
+                k<<<(unsigned)((past + kScWarps - 1) / kScWarps), 32 * kScWarps, smem, v->stream>>>(S);
+            }
+            if (past < S.ncell) {
+                constexpr size_t ls = sizeof(LightWarp<NCH>) * kLightWarps;
+                auto kl = k_scatter_light<KERNEL, NCH>;
+                GV_TRY(launch_smem(v, kl, ls, "scatter"));
+                GV_TRY(light_list(v, S.ncell, v->src_classes[NCH - 1]));
+                S.light_list = v->light_list.as<int32_t>();
+                kl<<<(unsigned)((S.ncell - past + kLightWarps - 1) / kLightWarps), 32 * kLightWarps, ls, v->stream>>>(S);
+            }
         }
     }
     // a cell with a dense cell among its 27 neighbours: at most 27 per dense cell
