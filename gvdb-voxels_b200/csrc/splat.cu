@@ -410,6 +410,62 @@ __device__ __forceinline__ void part_add(int32_t *acc, int idx, float x, float i
     atomicAdd(acc + CS + idx, lo);
 }
 
+// Position in a partial of extended-tile voxel (z * E + y) * E + x.
+template <int KERNEL>
+struct PartPos {
+    uint16_t pos[ExtTile<KERNEL>::E3];
+    constexpr PartPos() : pos() {
+        using X = ExtTile<KERNEL>;
+        for (int z = 0; z < X::E; z++)
+            for (int y = 0; y < X::E; y++)
+                for (int x = 0; x < X::E; x++) pos[(z * X::E + y) * X::E + x] = (uint16_t)X::part_index(x, y, z);
+    }
+};
+template <int KERNEL>
+__device__ constexpr PartPos<KERNEL> kPartPos{};
+
+__device__ __forceinline__ bool all_finite(float4 a) {
+    return isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w);
+}
+
+// Adds the points of a dense cell whose amounts are not all finite, which its sums
+// leave out, to its partial in memory, which the CTA has written, in bin order: one
+// warp, up to two taps a lane.  (ox, oy, oz): the extended tile's first voxel.
+// (k_scatter_rows has a loop of its own in sorted order: called there, this one cost
+// 30 us of 1.17 ms without such a point.)
+template <int KERNEL, int NCH>
+__device__ __forceinline__ void add_not_finite(const SplatArgs &S, uint32_t beg, uint32_t R, float *dst, int ox, int oy,
+                                               int oz) {
+    using T = Taps<KERNEL>;
+    using X = ExtTile<KERNEL>;
+    constexpr int N = T::N;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t i0 = 0; i0 < R; i0 += 32) {
+        unsigned left = __ballot_sync(0xffffffffu, i0 + lane < R && !all_finite(S.bin_amt[beg + min(i0 + lane, R - 1)]));
+        for (; left; left &= left - 1) {
+            const uint32_t p = beg + i0 + __ffs(left) - 1;
+            const float4 q = S.bin_pos[p], am = S.bin_amt[p];
+            const float a4[4] = {am.x, am.y, am.z, am.w};
+            const int32_t cloud = __float_as_int(q.w);
+            int3 o = make_int3(0, 0, 0);
+            if (cloud >= 0 && in_range(S.lim, cloud, S.lim.ncloud, 47))
+                o = make_int3(S.pos.origin[3 * cloud], S.pos.origin[3 * cloud + 1], S.pos.origin[3 * cloud + 2]);
+            float wx[N], wy[N], wz[N];
+            const int fx = T::eval_fine(q.x, wx) + o.x - ox, fy = T::eval_fine(q.y, wy) + o.y - oy,
+                      fz = T::eval_fine(q.z, wz) + o.z - oz;
+            if ((unsigned)fx > 8u || (unsigned)fy > 8u || (unsigned)fz > 8u) continue;
+            for (int t = lane; t < N * N * N; t += 32) {
+                const int tx = t % N, ty = t / N % N, tz = t / (N * N);
+                const float w = wx[tx] * wy[ty] * wz[tz];
+                const int pos = kPartPos<KERNEL>.pos[((fz + tz) * X::E + fy + ty) * X::E + fx + tx];
+#pragma unroll
+                for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] += a4[c] * w;
+            }
+            __syncwarp(); // the next point may reach the same voxels
+        }
+    }
+}
+
 // One work item per CTA: slice item.y of item.z of dense cell item.x
 // (item.w: the cell's accumulator slot when item.z > 1).  The partial goes
 // to part + cell_part[cell] * NCH * E3.
@@ -431,6 +487,7 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
     __shared__ double inv_s[NCH];
     __shared__ int32_t amax_bits[NCH]; // largest |amount| of the cell's points, as float bits
     __shared__ int last;
+    __shared__ int special; // some point's amounts are not all finite
     if (blockIdx.x >= S.cell_cnt[kCntWork]) return;
     const int4 item = S.part_work[blockIdx.x];
     const int64_t cell = item.x;
@@ -457,16 +514,23 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
     // the largest |amount| per channel over all the cell's points sets the
     // scale, the same in every slice of the cell
     if (threadIdx.x < NCH) amax_bits[threadIdx.x] = 0;
+    if (threadIdx.x == 0) special = 0;
+    bool finite = true;
     float mx[NCH];
 #pragma unroll
     for (int c = 0; c < NCH; c++) mx[c] = 0.0f;
     for (uint32_t j = threadIdx.x; j < R; j += kPartThreads) {
         const float4 a = S.bin_amt[beg + j];
+        if (!all_finite(a)) { // added after the sums
+            finite = false;
+            continue;
+        }
         const float a4[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
         for (int c = 0; c < NCH; c++) mx[c] = fmaxf(mx[c], fabsf(a4[c]));
     }
-    __syncthreads(); // amax_bits cleared
+    __syncthreads(); // amax_bits and special cleared
+    if (!finite) special = 1;
 #pragma unroll
     for (int c = 0; c < NCH; c++) {
         float x = mx[c];
@@ -514,7 +578,7 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
             const float a4[4] = {a.x, a.y, a.z, a.w};
             float s4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int c = 0; c < NCH; c++) s4[c] = ok ? a4[c] * scale[c] : 0.0f;
+            for (int c = 0; c < NCH; c++) s4[c] = ok && all_finite(a) ? a4[c] * scale[c] : 0.0f;
             pa[r] = make_float4(s4[0], s4[1], s4[2], s4[3]);
         }
         __syncthreads();
@@ -561,6 +625,11 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
         // |sum| < 2^53: exact in double; the power-of-two scalings are exact
         return (float)((double)(((long long)hi << L) + (long long)lo) * inv_s[c]);
     };
+    auto left_out = [&] { // the partial is written, by the whole CTA
+        if (!special) return;
+        __syncthreads();
+        if (warp == 0) add_not_finite<KERNEL, NCH>(S, beg, R, dst, ox, oy, oz);
+    };
     if (nslice == 1) {
         int c = 0, i0 = threadIdx.x;
         for (int i = threadIdx.x; i < NCH * X::E3; i += kPartThreads) {
@@ -568,6 +637,7 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
             dst[i] = value(c, acc[k], acc[k + X::CS]);
             if ((i0 += kPartThreads) >= X::E3) i0 -= X::E3, c++;
         }
+        left_out();
         return;
     }
     // a cell of several slices: this slice's integer sums into the cell's
@@ -599,6 +669,7 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
         if ((i0 += kPartThreads) >= X::E3) i0 -= X::E3, c++;
     }
     if (threadIdx.x == 0) S.part_done[item.w] = 0;
+    left_out();
 }
 
 // A voxel's channels side by side in a shared-memory tile: one access per tap
@@ -744,22 +815,6 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_rows(SplatArgs S, const i
         for (uint32_t p = p0; p < p1; p++) at += index[p] < mine;
         order[beg + at] = (int32_t)(beg + j);
     }
-}
-
-// Position in a cubic partial of extended-tile voxel z * 144 + y * 12 + x.
-struct PartPos {
-    uint16_t pos[ExtTile<GVDB2_KERNEL_CUBIC2>::E3];
-    constexpr PartPos() : pos() {
-        using X = ExtTile<GVDB2_KERNEL_CUBIC2>;
-        for (int z = 0; z < X::E; z++)
-            for (int y = 0; y < X::E; y++)
-                for (int x = 0; x < X::E; x++) pos[(z * X::E + y) * X::E + x] = (uint16_t)X::part_index(x, y, z);
-    }
-};
-__device__ constexpr PartPos kPartPos{};
-
-__device__ __forceinline__ bool all_finite(float4 a) {
-    return isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(a.w);
 }
 
 constexpr int kRowRec = 24; // floats a record: x weights twice each, 8 y weights, z weights, amounts
@@ -982,7 +1037,7 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
                     for (int c = 0; c < NCH; c++) sum[c] += g[c];
                 }
             }
-            const int pos = kPartPos.pos[z0 * X::E * X::E + v];
+            const int pos = kPartPos<GVDB2_KERNEL_CUBIC2>.pos[z0 * X::E * X::E + v];
 #pragma unroll
             for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] = sum[c];
         }
@@ -1011,7 +1066,7 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
             for (int t = lane; t < 64; t += 32) {
                 const int tx = t & 3, ty = (t >> 2) & 3, tz = t >> 4;
                 const float w = wx[tx] * wy[ty] * wz[tz];
-                const int pos = kPartPos.pos[((fz + tz) * X::E + fy + ty) * X::E + fx + tx];
+                const int pos = kPartPos<GVDB2_KERNEL_CUBIC2>.pos[((fz + tz) * X::E + fy + ty) * X::E + fx + tx];
 #pragma unroll
                 for (int c = 0; c < NCH; c++) dst[c * X::E3 + pos] += a4[c] * w;
             }
