@@ -214,29 +214,30 @@ __device__ __forceinline__ bool in_range(const SplatLimits &L, int64_t i, int64_
 constexpr uint32_t kSlicePts = 4096;
 // cell_cnt entries: huge, heavy, light cells; dense cells, dense work
 // items (slices), dense cells of more than one slice, dense cells listed for
-// k_scatter_rows, items of huge cells,
-// cells of each class of sources
+// k_scatter_rows, items of huge cells, cells of each class of sources, and the work
+// items of the cells listed for k_scatter_rows
 constexpr int kCntHuge = 0, kCntHeavy = 1, kCntLight = 2, kCntDense = 3, kCntWork = 4, kCntMulti = 5, kCntRows = 6,
-              kCntTiles = 7, kCntSrc = 8, kCntWords = 14;
-// Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic): 16.7M
-// points in cells of 1,024 on average, 4 channels, 1.18 + 0.15 ms (its sort)
-// against 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162
-// short units (a 300,000-point blob's cells of 512 to 700: 48 us against 20), more
-// make a cell its launch's tail.
-#ifndef GVDB2_ROWS_MIN
-#define GVDB2_ROWS_MIN 768
-#endif
-#ifndef GVDB2_ROWS_MAX
-#define GVDB2_ROWS_MAX 2048
-#endif
-constexpr int kRowsMin = GVDB2_ROWS_MIN, kRowsMax = GVDB2_ROWS_MAX;
+              kCntTiles = 7, kCntSrc = 8, kCntRowWork = 14, kCntWords = 15;
+// Dense cells of kRowsMin to kRowsMax points take k_scatter_rows (cubic) where a
+// volume has at least this many of them, by channels; else k_scatter_part.  16.7M
+// points in cells of 1,024 on average, 4 channels, 1.18 + 0.15 ms (its sort) against
+// 1.98 ms.  Fewer points a cell leave its two warps waiting on their 162 short units
+// (a 300,000-point blob's cells of 512 to 700: 48 us against 20), more make a cell its
+// launch's tail, and a cell's two warps take 0.2 us a point however idle the chip.  A
+// scatter of cells of 800 to 1,900 points with rows over one with fixed point only: 4
+// channels 0.99 to 1.19 at 300 to 600 cells, 0.83 to 0.90 at 800 to 1,500, 0.70 at
+// 8,000; 3 channels 1.04 to 1.14 at 600, 0.97 at 1,000; 2 channels 1.0 to 1.1 at 1,000,
+// 0.95 at 1,250; 1 channel, whose atomics are a quarter, 1.06 to 1.7 everywhere.
+constexpr int kRowsMin = 768, kRowsMax = 2048;
 static_assert(kRowsMax <= 65535, "16-bit positions in a cell");
+constexpr uint32_t kRowsCells[4] = {UINT32_MAX, 1200, 1000, 600};
+constexpr uint32_t kRowsLeast = 600;
 // A cell has an estimate of the points that reach it, dense cells' left out: its own
 // and, for the cubic (whose stencils reach 1.5 voxels past a face, of 8), 3/16 of
 // its face neighbours'.  The owner-computes pass takes the cells class by class, class
 // k having more than edge[k] and no more than edge[k - 1] (the last, the rest).
 constexpr int kSrcClasses = 6;
-static_assert(kCntSrc + kSrcClasses == kCntWords, "a count per class");
+static_assert(kCntSrc + kSrcClasses == kCntRowWork, "a count per class");
 struct SrcEdges {
     int edge[kSrcClasses - 1];
 };

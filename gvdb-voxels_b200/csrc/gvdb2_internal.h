@@ -215,6 +215,7 @@ struct Volume {
     // capacity, their keys' first positions (the sorted order itself is in
     // prank) and whether the scatter has sorted them since the binning
     DevBuf rows_list, row_off;
+    DevBuf row_work; // the same cells' work items, for scatters that sum them in fixed point
     int64_t rows_cap = 0;
     bool rows_sorted = false;
     // cells that hold points: heavy ones, light ones, items (cell, slice) of huge

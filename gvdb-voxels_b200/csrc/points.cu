@@ -148,7 +148,7 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // cells: each gets a partial slot (part[c], -1 for the other cells), ceil(k / slice) work items (cell,
 // slice, slices, accumulator slot) and, when that is more than one, an accumulator
 // slot for its integer sums.  With rows_on the dense cells of kRowsMin to kRowsMax
-// points are listed in `rows` instead of the work items.  cls gets each
+// points are listed in `rows`, and their items apart in row_work.  cls gets each
 // cell's class of sources (SrcEdges), blk[k * gridDim.x + b] how many of block b's
 // cells are in class k, cnt[kCntSrc + k] how many of all.  Cells of at most `light` (<=
 // kLightCell) points are light.  All of it depends on the cell and its neighbours
@@ -156,7 +156,7 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // reg_off holds each (cell, region) bin's first entry; off[c] = reg_off[27 c], each
 // cell's (c = ncell: the end), is written for the kernels that follow.
 __global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int2 *tiles,
-                            int32_t *part, int32_t *rows, int4 *work, uint32_t *cnt, const int32_t *nbr27, int m,
+                            int32_t *part, int32_t *rows, int4 *work, int4 *row_work, uint32_t *cnt, const int32_t *nbr27, int m,
                             uint32_t dense_min, uint32_t slice, uint32_t light_max, bool cubic, bool rows_on,
                             uint8_t *cls, SrcEdges E, uint32_t *blk) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -228,11 +228,12 @@ __global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncel
     const bool row = rows_on && dense && k >= (uint32_t)kRowsMin && k <= (uint32_t)kRowsMax;
     const unsigned rn = __ballot_sync(0xffffffffu, row);
     if (row) rows[warp_agg_inc(cnt, (uint32_t)kCntRows, rn)] = (int32_t)c;
-    if (dense && !row) {
+    if (dense) {
         const uint32_t ns = (k + slice - 1) / slice;
-        const uint32_t first = atomicAdd(cnt + kCntWork, ns);
+        const uint32_t first = atomicAdd(cnt + (row ? kCntRowWork : kCntWork), ns);
         const int32_t acc = ns > 1 ? (int32_t)atomicAdd(cnt + kCntMulti, 1u) : -1;
-        for (uint32_t i = 0; i < ns; i++) work[first + i] = make_int4((int32_t)c, (int32_t)i, (int32_t)ns, acc);
+        for (uint32_t i = 0; i < ns; i++)
+            (row ? row_work : work)[first + i] = make_int4((int32_t)c, (int32_t)i, (int32_t)ns, acc);
     }
 }
 
@@ -590,6 +591,7 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
     v->work_cap = dmin > 0 ? v->dense_cap + n / sl : 0;
     v->multi_cap = std::min<int64_t>(v->dense_cap, n / (sl + 1));
     GV_CUDA(v, v->rows_list.ensure(sizeof(int32_t) * (size_t)std::max<int64_t>(v->rows_cap, 1), s));
+    GV_CUDA(v, v->row_work.ensure(sizeof(int4) * (size_t)std::max<int64_t>(v->rows_cap > 0 ? v->rows_cap + n / sl : 0, 1), s));
     GV_CUDA(v, v->part_work.ensure(sizeof(int4) * (size_t)std::max<int64_t>(v->work_cap, 1), s));
     v->heavy_grid = v->light_grid = 0;
     v->src_cells.fill(-1);
@@ -601,7 +603,8 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
         GV_CUDA(v, v->cell_blk.ensure(sizeof(uint32_t) * (2 * kSrcClasses * (size_t)g + 1), s));
         k_cell_list<<<g, kListCells, 0, s>>>(v->reg_off.as<uint32_t>(), v->bin_off.as<uint32_t>(), nbins, v->cell_list.as<int32_t>(),
                                       v->cell_light.as<int32_t>(), v->cell_tiles.as<int2>(),
-                                      v->cell_part.as<int32_t>(), v->rows_list.as<int32_t>(), v->part_work.as<int4>(), v->cell_cnt.as<uint32_t>(),
+                                      v->cell_part.as<int32_t>(), v->rows_list.as<int32_t>(), v->part_work.as<int4>(), v->row_work.as<int4>(),
+                                      v->cell_cnt.as<uint32_t>(),
                                       v->nbr27.as<int32_t>(), m, (uint32_t)dmin, (uint32_t)v->tune_slice, (uint32_t)v->tune_light,
                                       cubic, rows, v->cell_cls.as<uint8_t>(), few ? kSrcEdgesOne[cubic] : kSrcEdges[cubic],
                                       v->cell_blk.as<uint32_t>());
@@ -628,7 +631,7 @@ gvdb2_status bin_points(Volume *v, int kernel, int n, const float trans[3]) {
             v->light_grid = cw[kCntLight];
             v->dense_cap = cw[kCntDense];
             v->rows_cap = cw[kCntRows];
-            v->work_cap = cw[kCntWork];
+            v->work_cap = (int64_t)cw[kCntWork] + cw[kCntRowWork];
             v->multi_cap = cw[kCntMulti];
             const bool sparse = 2 * (int64_t)cw[kCntSrc + kSrcClasses - 1] >= nbins;
             for (int i = 0; i < 4; i++) {

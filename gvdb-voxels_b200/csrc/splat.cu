@@ -233,7 +233,8 @@ struct SplatArgs {
     uint32_t slice; // points per dense-cell work item
     SplatLimits lim;
     const int32_t *cell_part;
-    const int4 *part_work;
+    const int4 *part_work, *row_work;
+    uint32_t rows_cells; // as few row cells as take k_scatter_rows
     float *part;
     int32_t *part_acc;
     uint32_t *part_done;
@@ -488,8 +489,11 @@ __global__ void __launch_bounds__(kPartThreads) k_scatter_part(SplatArgs S) {
     __shared__ int32_t amax_bits[NCH]; // largest |amount| of the cell's points, as float bits
     __shared__ int last;
     __shared__ int special; // some point's amounts are not all finite
-    if (blockIdx.x >= S.cell_cnt[kCntWork]) return;
-    const int4 item = S.part_work[blockIdx.x];
+    // the work items, and those of the row cells where these are too few for k_scatter_rows
+    const uint32_t items = S.cell_cnt[kCntWork];
+    const bool rest = blockIdx.x >= items;
+    if (rest && (S.cell_cnt[kCntRows] >= S.rows_cells || blockIdx.x - items >= S.cell_cnt[kCntRowWork])) return;
+    const int4 item = rest ? S.row_work[blockIdx.x - items] : S.part_work[blockIdx.x];
     const int64_t cell = item.x;
     const int nslice = item.z;
     // every check below is the same for the whole CTA
@@ -756,7 +760,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_rows(SplatArgs S, const i
     __shared__ uint16_t place[kRowsMax];
     __shared__ uint8_t key[kRowsMax];
     static_assert(kRowKeys <= 256, "8-bit keys");
-    if (blockIdx.x >= S.cell_cnt[kCntRows]) return;
+    if (blockIdx.x >= S.cell_cnt[kCntRows] || S.cell_cnt[kCntRows] < kRowsLeast) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t cell = list[blockIdx.x];
     if (!in_range(S.lim, cell, S.ncell, 30)) return; // the same for the whole CTA
@@ -837,7 +841,7 @@ __global__ void __launch_bounds__(64) k_scatter_rows(SplatArgs S, const int32_t 
     constexpr int NP = (NCH + 1) / 2; // channel pairs (one channel: its value twice is not needed, .x only)
     extern __shared__ __align__(16) unsigned char row_smem[];
     RowSmem<NCH> &M = *reinterpret_cast<RowSmem<NCH> *>(row_smem);
-    if (blockIdx.x >= S.cell_cnt[kCntRows]) return;
+    if (blockIdx.x >= S.cell_cnt[kCntRows] || S.cell_cnt[kCntRows] < S.rows_cells) return;
     const int lane = threadIdx.x & 31, half = threadIdx.x >> 5;
     const int64_t cell = list[blockIdx.x];
     if (!in_range(S.lim, cell, S.ncell, 35)) return; // the same for the whole CTA
@@ -2525,6 +2529,8 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     S.dense_cap = v->dense_cap;
     S.multi_cap = v->multi_cap;
     S.slice = (uint32_t)v->tune_slice;
+    S.row_work = v->row_work.as<int4>();
+    S.rows_cells = KERNEL == GVDB2_KERNEL_CUBIC2 ? kRowsCells[NCH - 1] : UINT32_MAX;
     // the list's count sits in its last 16 bytes
     S.merge_cnt = reinterpret_cast<uint32_t *>(v->merge_list.as<char>() + v->merge_list.bytes - 16);
     S.merge_list = v->merge_list.as<int32_t>();
@@ -2535,7 +2541,7 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     if (v->bin_key.n > 0)
         k_pack_amounts<NCH><<<grid_for(v->bin_key.n, 256, 1ll << 31), 256, 0, v->stream>>>(S);
     if constexpr (KERNEL == GVDB2_KERNEL_CUBIC2) {
-        if (v->rows_cap > 0) {
+        if (v->rows_cap >= S.rows_cells) {
             auto kr = k_scatter_rows<NCH>;
             GV_TRY(launch_smem(v, kr, sizeof(RowSmem<NCH>), "scatter"));
             kr<<<(unsigned)v->rows_cap, 64, sizeof(RowSmem<NCH>), v->stream>>>(
@@ -2593,7 +2599,7 @@ SplatArgs channel_group(const SplatArgs &S, int first, int count) {
 // The dense cells' points in row order, once per binning.  prank, the ranks
 // that the binning is done with, holds the order.
 gvdb2_status sort_rows(Volume *v, const SplatArgs &S0) {
-    if (v->rows_sorted || v->rows_cap == 0) return GVDB2_OK;
+    if (v->rows_sorted || v->rows_cap < kRowsCells[std::min(S0.nch, 4) - 1]) return GVDB2_OK;
     GV_CUDA(v, v->row_off.ensure(sizeof(uint16_t) * kRowOff * (size_t)v->dense_cap, v->stream));
     SplatArgs S = S0;
     S.dense_cap = v->dense_cap;

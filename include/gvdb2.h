@@ -333,9 +333,10 @@ GVDB2_API gvdb2_status gvdb2_gather_kernel_backward(gvdb2_volume *v, int kernel,
  * Launch settings of the kernel splats and gathers.  dense: cells of at
  * least this many points take the scatter's partial-sum path (a CTA per
  * slice staging the cell's extended tile in shared memory; outside
- * deterministic mode the cubic splat sums dense cells of 768 to 2,048 points in
- * registers instead), the other cells the owner-computes warps; 0 sends every cell to the owner warps (0 or
- * [128, 2^24]).  slice: points per CTA of a dense cell (a multiple of 128 in
+ * deterministic mode the cubic splat of 2 to 4 channels sums dense cells of 768
+ * to 2,048 points in registers instead, in volumes of 600 of them and more), the
+ * other cells the owner-computes warps; 0 sends every cell to the owner warps
+ * (0 or [128, 2^24]).  slice: points per CTA of a dense cell (a multiple of 128 in
  * [128, 65536]).  light: cells of at most this many points are gathered a
  * warp per cell, a lane per point, with taps read from the atlas; the others
  * through a halo tile staged in shared memory (0..32).  Defaults 512, 4096,
