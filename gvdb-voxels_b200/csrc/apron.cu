@@ -12,56 +12,64 @@
 //     neighbour table of UpdateNeighbors (V:2527-2556).  A missing
 //     neighbour is -1 here; the reference stores 0xFFFF and then fails to
 //     recognise it (O:51).
-#include <algorithm>
 #include <vector>
 
 #include "dev_common.cuh"
-
 
 namespace gvdb2 {
 
 namespace {
 
 struct ApronChans {
-    float *chan[4];
+    float *chan[kMaxChan];
+    int nch;
 };
 
-// One CTA per slot, NC channels of the call.  `list` holds, in tile order, every
-// apron voxel of a tile: its tile offset and the neighbour k (0..26) that owns it
-// with the offset of the owner's interior voxel, so the kernel does no index
-// arithmetic.  Bound by the latency of its scattered reads (an x face's voxels lie
-// a row apart) and by the sectors that they and the writes touch: a thread takes
-// EN entries at a time, all of their reads issued before the first write.  One
-// channel of 612k bricks of 8^3: 1.52 ms with 2 entries, loops over up to 4
-// channels and the neighbours staged in shared memory behind a barrier, 1.19 with
-// 2 entries without these, 1.08 with 4, 1.10 with 8.
-constexpr int kApronThreads = 128;
-template <int NC> struct ApronEntries { static constexpr int n = NC <= 2 ? 4 : 2; };
-template <int NC>
-__global__ void __launch_bounds__(kApronThreads) k_apron(ApronChans C, const int32_t *nbr27, const int2 *list, int nlist,
+// One CTA per slot, group of NC of the call's channels (GROUPS: of several, the last
+// of fewer) and kApronChunk entries of `list`, one chunk for bricks of 8^3, 7 for
+// 32^3.  `list` holds, in tile order, every apron voxel of a tile: its tile offset and
+// the neighbour k (0..26) that owns it with the offset of the owner's interior voxel,
+// so the kernel does no index arithmetic.  Bound by the latency of its scattered
+// reads (an x face's voxels lie a row apart) and by the sectors that they and the
+// writes touch: a thread takes EN entries at a time, all of their reads issued before
+// the first write.  One channel of 612k bricks of 8^3: 1.52 ms with 2 entries, loops
+// over up to 4 channels and the neighbours staged in shared memory behind a barrier,
+// 1.19 with 2 entries without these, 1.08 with 4, 1.10 with 8.  1 and 2 channels 128
+// threads of 4 entries, 3 and 4 channels 256 of 2: 19,683 bricks of 8^3, 4 channels
+// 145 us with 128, 137 with 256 (bricks of 4^3 have 152 entries: 128).  8 channels of
+// 216 bricks of 8^3 13 us, of 27 of 32^3 25, of 8 of 64^3 25; with a launch a group and
+// a CTA a slot 18, 76 and 233.
+constexpr int kApronChunk = 1024;
+template <int NC> struct ApronShape { static constexpr int entries = NC <= 2 ? 4 : 2, threads = NC <= 2 ? 128 : 256; };
+template <int NC, bool GROUPS>
+__global__ void __launch_bounds__(ApronShape<NC>::threads) k_apron(ApronChans C, const int32_t *nbr27, const int2 *list, int nlist,
                                                          int64_t tvox, float boundval) {
-    constexpr int EN = ApronEntries<NC>::n;
+    constexpr int EN = ApronShape<NC>::entries;
+    const int threads = blockDim.x;
     const int64_t slot = blockIdx.x;
+    const int first = GROUPS ? blockIdx.y * NC : 0, chans = GROUPS ? C.nch - first : NC;
     const int32_t *nbs = nbr27 + slot * 27;
-    for (int i = threadIdx.x; i < nlist; i += EN * kApronThreads) {
+    const int end = min(nlist, ((int)blockIdx.z + 1) * kApronChunk);
+    for (int i = blockIdx.z * kApronChunk + threadIdx.x; i < end; i += EN * threads) {
         int2 e[EN];
         int32_t nb[EN];
         float val[EN][NC];
 #pragma unroll
-        for (int k = 0; k < EN; k++) e[k] = __ldg(list + min(i + k * kApronThreads, nlist - 1));
+        for (int k = 0; k < EN; k++) e[k] = __ldg(list + min(i + k * threads, end - 1));
 #pragma unroll
         for (int k = 0; k < EN; k++) nb[k] = __ldg(nbs + (e[k].y >> 24));
 #pragma unroll
         for (int k = 0; k < EN; k++) {
             const int64_t src = (int64_t)nb[k] * tvox + (e[k].y & 0xFFFFFF);
 #pragma unroll
-            for (int c = 0; c < NC; c++) val[k][c] = nb[k] >= 0 ? __ldcg(C.chan[c] + src) : boundval;
+            for (int c = 0; c < NC; c++) val[k][c] = nb[k] >= 0 && c < chans ? __ldcg(C.chan[first + c] + src) : boundval;
         }
 #pragma unroll
         for (int k = 0; k < EN; k++)
-            if (i + k * kApronThreads < nlist)
+            if (i + k * threads < end)
 #pragma unroll
-                for (int c = 0; c < NC; c++) C.chan[c][slot * tvox + e[k].x] = val[k][c];
+                for (int c = 0; c < NC; c++)
+                    if (c < chans) C.chan[first + c][slot * tvox + e[k].x] = val[k][c];
     }
 }
 
@@ -122,26 +130,24 @@ gvdb2_status apron_list(Volume *v) {
 gvdb2_status update_apron(Volume *v, int chan, float boundval) {
     if (v->apron == 0) return GVDB2_OK; // V:4421
     if (!v->atlas_valid) return fail(v, GVDB2_ERR_STATE, "UpdateAtlas must follow the topology rebuild");
-    float *chans[kMaxChan];
-    int nch = 0;
+    ApronChans C{};
     for (int c = 0; c < kMaxChan; c++) {
         if (chan >= 0 && c != chan) continue;
         if (!v->has_chan[c]) {
             if (chan >= 0) return fail(v, GVDB2_ERR_ARG, "bad channel");
             continue;
         }
-        chans[nch++] = v->atlas[c].as<float>();
+        C.chan[C.nch++] = v->atlas[c].as<float>();
     }
-    if (v->atlas_last == 0 || nch == 0) return GVDB2_OK;
+    if (v->atlas_last == 0 || C.nch == 0) return GVDB2_OK;
     GV_TRY(apron_list(v));
-    for (int first = 0; first < nch; first += 4) {
-        const int n = std::min(4, nch - first);
-        ApronChans C{};
-        for (int c = 0; c < n; c++) C.chan[c] = chans[first + c];
-        auto k = n == 1 ? k_apron<1> : (n == 2 ? k_apron<2> : (n == 3 ? k_apron<3> : k_apron<4>));
-        k<<<(unsigned)v->atlas_last, kApronThreads, 0, v->stream>>>(C, v->nbr27.as<int32_t>(), v->apron_list.as<int2>(),
-                                                                    v->apron_list_n, v->tile_vox(), boundval);
-    }
+    const int groups = (C.nch + 3) / 4, n = (C.nch + groups - 1) / groups; // even groups
+    auto k = groups > 1 ? (n == 3 ? k_apron<3, true> : k_apron<4, true>)
+                        : (n == 1 ? k_apron<1, false> : (n == 2 ? k_apron<2, false> : (n == 3 ? k_apron<3, false> : k_apron<4, false>)));
+    const dim3 grid((unsigned)v->atlas_last, (unsigned)groups, (unsigned)((v->apron_list_n + kApronChunk - 1) / kApronChunk));
+    const int threads = n <= 2 || v->apron_list_n <= 256 ? ApronShape<1>::threads : ApronShape<4>::threads;
+    k<<<grid, threads, 0, v->stream>>>(
+        C, v->nbr27.as<int32_t>(), v->apron_list.as<int2>(), v->apron_list_n, v->tile_vox(), boundval);
     GV_CUDA(v, cudaGetLastError());
     return GVDB2_OK;
 }
