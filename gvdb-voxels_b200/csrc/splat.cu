@@ -2391,12 +2391,25 @@ __device__ __forceinline__ void gather_light_cells(const GatherArgs &G, int64_t 
     }
 }
 
+// CTAs of k_gather_tile an SM that the registers are kept down for (0: as they come).
+// 4M points, 60 to 4,000 a cell, time over that of the sums tap by tap: position
+// gradient of a cubic gather, 3 channels, 1.00 to 1.08 at 75 registers, 0.97 to 1.04 at
+// 64; cubic gather, 4 channels, 0.92 to 1.08 at 56, 0.90 to 1.02 at 48; tent scatter's
+// adjoint, 4 channels, 0.93 to 1.15 at 72, 0.97 to 1.06 at 64; the cubic's, 2 channels,
+// 0.89 to 1.09 at 72, 0.90 to 0.97 at 64, and 3 channels 0.86 to 1.02 at 80, 0.87 to
+// 1.20 without.
+constexpr int gather_tile_blocks(int kernel, int mode, int nch) {
+    const bool cubic = kernel == GVDB2_KERNEL_CUBIC2;
+    if (mode == kScatterBwd) return nch == 4 ? (cubic ? 3 : 4) : (nch == 3 ? 3 : (nch == 2 && cubic ? 4 : 0));
+    if (!cubic) return 0;
+    return mode == kGatherBwd ? (nch == 3 ? 4 : 0) : (nch == 4 ? 5 : 0);
+}
 // Two launches: a halo tile per item or heavy cell (every cell, in cell
 // order, when no cell list is given), then the light cells, kLightPack a warp.
 // One fused launch measured slower: the light path's registers (66) halved
 // the tiles' occupancy.
 template <int KERNEL, int MODE, int NCH>
-__global__ void __launch_bounds__(kGatherThreads, MODE == kScatterBwd && NCH >= 3 ? 3 : 0) k_gather_tile(GatherArgs G) {
+__global__ void __launch_bounds__(kGatherThreads, gather_tile_blocks(KERNEL, MODE, NCH)) k_gather_tile(GatherArgs G) {
     gather_tile_cell<KERNEL, MODE, NCH>(G, blockIdx.x);
 }
 // The register budgets are measured: batched clouds (one channel) forward and two
