@@ -308,7 +308,6 @@ struct ScArgs {
     int sc, scdim, scpb;
     int64_t num_sc;
     LeafLookup L;
-    const Node *leaves;
     int64_t nleaves;
     const uint32_t *mapping; // a leaf's place among the listed ones (nullptr: its pool index)
     // pass 2 (InsertPointsSubcell_FP16): quantization ranges, velocities
@@ -333,9 +332,12 @@ __device__ __forceinline__ uint16_t quantize16(float x, float lo, float range) {
 // reference; an insert never writes past the counted capacity of its
 // subcell.  Bound by an atomic add a visit and, in the inserts, by the 12-byte
 // entries they place.  The box's leaves are looked up once a brick, at most two
-// an axis, and not once a subcell: 4.2M points, 47.8M visits, 461 + 685 -> 321 +
-// 581 us to count and insert.  (Brick by brick, the lanes' loops diverge: 361 +
-// 683.  One add for the lanes of a warp that visit a subcell together: 508 + 938.)
+// an axis, and not once a subcell: 3M points at random, 64 a cell, 4^3 subcells and
+// radius 2, 686 + 1,798 -> 329 + 1,574 us to count and insert; in cell order 498 + 624
+// -> 266 + 512.  (Three subcells' adds along z before the first entry: 377 + 1,563 and
+// 295 + 499, but 8^3 subcells 306 + 434 instead of 258 + 400.  Brick by brick, the
+// lanes' loops diverge, and one add for the lanes of a warp that visit a subcell
+// together was slower by half.)
 template <int PASS>
 __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *off, float *pnt) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -427,22 +429,12 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *off, float *
             const bool y1 = (sy >> lr) != by;
             const int64_t h0 = y1 ? g10 : g00, h1 = y1 ? g11 : g01;
             const int row = ((sy & rm) >> ls) * A.scdim + ((sx & rm) >> ls);
-            // three along z at a time, their adds before the first entry is placed
-            for (int sz0 = mn[2]; sz0 <= mx[2]; sz0 += 3 * A.sc) {
-                int64_t idx[3];
-                uint32_t o[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    const int sz = sz0 + k * A.sc;
-                    const int64_t h = (sz >> lr) != bz ? h1 : h0;
-                    idx[k] = h + ((sz & rm) >> ls) * (A.scdim * A.scdim) + row;
-                    if (sz > mx[2] || h < 0 || idx[k] >= A.num_sc) idx[k] = -1;
-                    if (idx[k] >= 0) o[k] = atomicAdd(&cnt[idx[k]], 1u);
-                }
-                if (PASS != 0)
-#pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (idx[k] >= 0) place(idx[k], o[k]);
+            for (int sz = mn[2]; sz <= mx[2]; sz += A.sc) {
+                const int64_t h = (sz >> lr) != bz ? h1 : h0;
+                const int64_t idx = h + ((sz & rm) >> ls) * (A.scdim * A.scdim) + row;
+                if (h < 0 || idx >= A.num_sc) continue;
+                const uint32_t o = atomicAdd(&cnt[idx], 1u);
+                if (PASS != 0) place(idx, o);
             }
         }
     }
@@ -697,7 +689,6 @@ gvdb2_status insert_points_subcell(Volume *v, int sc, int n, float radius, const
     A.scpb = scpb;
     A.num_sc = num_sc;
     A.L = make_lookup(v);
-    A.leaves = v->pool_ptr(0);
     A.nleaves = nmap;
     A.mapping = mapping;
     A.pmin = make_float3(v->posmin[0], v->posmin[1], v->posmin[2]); // mPosMin, mPosRange (V:5452-5462)
