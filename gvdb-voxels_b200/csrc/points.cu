@@ -367,8 +367,9 @@ __global__ void k_sc_visit(ScArgs A, uint32_t *cnt, const uint32_t *off, float *
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         mn[a] = max(((int)(w[a] - A.radius) / A.sc) * A.sc, 0);
-        mx[a] = ((int)(w[a] + 1 + A.radius) / A.sc) * A.sc;
-        if (mx[a] < 0) return;
+        // no brick lies past 2^30; a box there would step past the largest int
+        mx[a] = (min((int)(w[a] + 1 + A.radius), 1 << 30) / A.sc) * A.sc;
+        if (mx[a] < mn[a]) return;
     }
     const int lr = A.L.g.log2r0, rm = (1 << lr) - 1, ls = __ffs(A.sc) - 1; // a power of two, as it divides the brick
     // first subcell of a brick's subcells, or -1
