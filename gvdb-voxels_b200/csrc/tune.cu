@@ -10,10 +10,12 @@
 //           with taps read from the atlas, the others through a staged halo
 //           tile -- the gather's tile staging.
 // A candidate is timed with CUDA events on the volume's stream, on the
-// caller's own call (median of three after an untimed run that also bins);
+// caller's own call (median of three after an untimed run that also bins; each
+// run sorts the row cells anew, as a scatter on fresh bins does);
 // the fastest stays on the volume and goes to the cache under the call's
-// workload class: device name and SM count, operation, kernel, channels,
-// brick width and the points per active 8^3 cell rounded to a power of two.
+// workload class: device name and SM count, operation, kernel, channels, brick
+// width, the points per active 8^3 cell rounded to a power of two, and the
+// generation of the kernels (a setting timed with earlier ones is not taken).
 // With GVDB2_OPT_AUTOTUNE set, every kernel splat and gather looks its
 // class up first and takes a cached setting when there is one.
 //
@@ -49,6 +51,7 @@ struct Entry {
 };
 
 std::mutex g_cache_mu;
+constexpr int kGeneration = 3; // of the splat kernels that the settings are for
 
 bool parse_line(const std::string &line, std::string &key, Entry &e) {
     const size_t tab = line.find('\t');
@@ -150,7 +153,7 @@ std::string tune_key(Volume *v, const char *op, int kernel, int nch, int64_t n) 
     const double cells = (double)std::max<int64_t>(1, v->atlas_last) * m * m * m;
     const int dens = (int)std::lround(std::log2(std::max(1.0, (double)n / cells)));
     char b[320];
-    std::snprintf(b, sizeof(b), "%s|%s|k%d|c%d|r%d|d%d", dev.c_str(), op, kernel, nch, v->res(0), dens);
+    std::snprintf(b, sizeof(b), "%s|%s|k%d|c%d|r%d|d%d|g%d", dev.c_str(), op, kernel, nch, v->res(0), dens, kGeneration);
     for (char *c = b; *c; c++)
         if (*c == '\t' || *c == '\n') *c = ' ';
     return b;
@@ -213,6 +216,7 @@ gvdb2_status autotune(Volume *v, const char *op, int kernel, int nch, int64_t n,
         if ((st = call()) != GVDB2_OK) break; // untimed: bins with this candidate's cell lists
         float t[3];
         for (int r = 0; r < 3 && st == GVDB2_OK; r++) {
+            v->rows_sorted = false;
             cudaEventRecord(e0, v->stream);
             st = call();
             cudaEventRecord(e1, v->stream);
