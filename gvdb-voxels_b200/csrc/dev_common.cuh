@@ -186,10 +186,7 @@ constexpr uint32_t kLightCell = 32;
 constexpr uint32_t kTilePts = 2048;
 // Cells of at least kDenseCell points are splatted into partial sums (the
 // scatter's dense path), kSlicePts points per CTA.
-#ifndef GVDB2_DENSE_CELL
-#define GVDB2_DENSE_CELL 512
-#endif
-constexpr uint32_t kDenseCell = GVDB2_DENSE_CELL;
+constexpr uint32_t kDenseCell = 512;
 
 // Sizes the splat kernels check their data-derived indices against: an
 // index out of range (bins inconsistent with the topology) skips the access

@@ -1446,14 +1446,9 @@ __global__ void __launch_bounds__(32 * kLightWarps) k_scatter_light(SplatArgs S)
 // The adds happen in the order of the sources (the bins) and of the stable
 // sort, then k_scatter_merge adds the partials in a fixed order, so with
 // deterministic binning the result is bit-reproducible.
-#ifndef GVDB2_SC_CAP
-#define GVDB2_SC_CAP 128
-#endif
-#ifndef GVDB2_SC_MIN_BLOCKS
-#define GVDB2_SC_MIN_BLOCKS 4
-#endif
-constexpr int kScWarps = 4;                    // cells per CTA
-constexpr int kScCap = GVDB2_SC_CAP;           // records per chunk
+constexpr int kScWarps = 4;     // cells per CTA
+constexpr int kScMinBlocks = 4; // CTAs an SM
+constexpr int kScCap = 128;     // records per chunk
 
 struct ScChunk {
     // x weights on the cell's voxel columns 0..7: half q (columns 4q..4q+3)
@@ -1518,9 +1513,6 @@ __device__ __forceinline__ void sc_sort_chunk(ScChunk &C, int fill, int lane) {
     __syncwarp();
 }
 
-#ifndef GVDB2_SC_PIPE
-#define GVDB2_SC_PIPE 0
-#endif
 // A record's values that lane (y, q) reads.
 struct ScRec {
     float4 xv; // x weights on columns 4q..4q+3
@@ -1531,23 +1523,11 @@ struct ScRec {
 __device__ __forceinline__ ScRec sc_load(const ScChunk &C, int r, int y, int q) {
     return ScRec{C.xw[r][q ^ (r & 1)], C.wy[r][y], C.wz[r], C.am[r]};
 }
-// Visits the sorted chunk's records i in [lo, hi) in order; with
-// GVDB2_SC_PIPE the next record's values are read while the current one is
-// added.
+// Visits the sorted chunk's records i in [lo, hi) in order.  (With the next record's
+// values read while the current one is added: no faster.)
 template <class Visit>
 __device__ __forceinline__ void sc_walk(const ScChunk &C, int lo, int hi, int y, int q, const Visit &visit) {
-    if (GVDB2_SC_PIPE) {
-        if (lo >= hi) return;
-        ScRec cur = sc_load(C, C.order[lo], y, q);
-        for (int i = lo; i < hi; i++) {
-            ScRec nxt = cur;
-            if (i + 1 < hi) nxt = sc_load(C, C.order[i + 1], y, q);
-            visit(cur);
-            cur = nxt;
-        }
-    } else {
-        for (int i = lo; i < hi; i++) visit(sc_load(C, C.order[i], y, q));
-    }
+    for (int i = lo; i < hi; i++) visit(sc_load(C, C.order[i], y, q));
 }
 
 // Adds the chunk's records that reach the voxels of lane (y, q, h)'s group:
@@ -1628,11 +1608,8 @@ __device__ __forceinline__ void sc_accumulate_cp(const ScChunk &C, float2 (&acc)
     }
 }
 
-#ifndef GVDB2_SC_CHPAIR
-#define GVDB2_SC_CHPAIR 1
-#endif
 // Channel pairs for 2 to 4 channels, x pairs for one channel.
-template <int NCH> struct ScLayout { static constexpr bool kChPairs = GVDB2_SC_CHPAIR && NCH > 1; };
+template <int NCH> struct ScLayout { static constexpr bool kChPairs = NCH > 1; };
 
 // One cell, by one warp.
 template <int KERNEL, int NCH>
@@ -1861,7 +1838,7 @@ __device__ __forceinline__ void scatter_cell(const SplatArgs &S, ScChunk &C, int
 
 // kScWarps listed cells per CTA, a warp per cell.
 template <int KERNEL, int NCH>
-__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_cells(SplatArgs S) {
+__global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_cells(SplatArgs S) {
     extern __shared__ __align__(16) unsigned char sc_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = (int64_t)blockIdx.x * kScWarps + warp;
@@ -1881,7 +1858,7 @@ constexpr size_t owner_warp_bytes() {
     return std::max(sizeof(ScChunk), sizeof(LightWarp<NCH>));
 }
 template <int KERNEL, int NCH>
-__global__ void __launch_bounds__(32 * kScWarps, GVDB2_SC_MIN_BLOCKS) k_scatter_owner(SplatArgs S) {
+__global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_owner(SplatArgs S) {
     constexpr size_t share = owner_warp_bytes<NCH>();
     static_assert(share % 16 == 0, "16-byte accesses");
     extern __shared__ __align__(16) unsigned char sc_smem[];
