@@ -551,9 +551,9 @@ def run_ours(a):
 # launch moves about this many bytes x bricks.
 TRAFFIC_PER_BRICK = {
     # k_sort_rows, k_pack_amounts, k_scatter_rows, k_scatter_owner, k_scatter_merge
-    "scatter": ((33.9 + 0.4) + (33.6 + 0.3) + (76.3 + 11.4) + (9.9 + 8.4) + (88.8 + 5.3)) * 1e6 / 3240,
+    "scatter": ((41.9 + 0.1) + (33.6 + 0.2) + (76.1 + 11.4) + (9.6 + 8.2) + (88.5 + 4.8)) * 1e6 / 3240,
     # k_gather_tile, k_gather_light
-    "gather": ((71.4 + 3.7) + (12.4 + 0.0)) * 1e6 / 3240,
+    "gather": ((71.4 + 3.5) + (12.4 + 0.0)) * 1e6 / 3240,
 }
 TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 2,097,152-point block at the "
                   "16,777,216-point step's density, scaled by bricks")

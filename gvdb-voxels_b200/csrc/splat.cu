@@ -705,19 +705,19 @@ __device__ __forceinline__ void gvec_get(const typename GVec<NCH>::T &v, float *
 // first rows (y0 in [0, 4] or [5, 8]) and one first plane z0 in [0, 8], each in
 // order of the first column x0.  A warp per half takes its units in order of
 // z0: lane (y, z) holds target row y of the half's 8 and target plane z0 + z,
-// and keeps the 4 columns a stencil covers in registers, a window that moves
-// along x; a column that the window leaves is added to the half's planes in
+// and keeps the 4 columns a stencil covers in registers, two windows that move
+// along x; a column that the windows leave is added to the half's planes in
 // shared memory, which hold 4 planes in turn.  After plane z0's last unit its
 // rows, the two halves' sums together, go to the partial.
 //
 // Per point and channel pair a lane adds 4 products (packed FMAs), half of
 // them zero (4 of the 8 rows): bound by instruction issue and by the latency
-// of the records' reads (43% of issue slots with 14 warps an SM; shared memory
+// of the records' reads (50% of issue slots with 15 warps an SM; shared memory
 // for 20 KB a cell bounds them: with a fifth plane, which spares a barrier a
 // plane, 24 KB and 1.22 ms instead of 1.15 for 16.7M points, one window).  The
-// loop over first columns is not unrolled: its 9 copies cost 0.4 ms more.  The fixed-point atomics
-// of k_scatter_part, two per tap and channel, are bound by the shared-memory
-// atomic rate, 30 of 32 lanes a cycle.
+// loop over first columns is not unrolled: its 9 copies cost 0.4 ms more.  The
+// fixed-point atomics of k_scatter_part, two per tap and channel, are bound by
+// the shared-memory atomic rate, 30 of 32 lanes a cycle.
 //
 // Sums are float, in two windows that take every other point.  However the
 // points lie, a register takes at most kRowFold / 2 terms a first column, 4 of
