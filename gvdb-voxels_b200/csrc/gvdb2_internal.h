@@ -208,6 +208,10 @@ struct Volume {
     // the cells of k_scatter_light in cell order
     DevBuf cell_owner, cell_cls, cell_blk, light_list;
     bool ordered = false; // cell_owner is made
+    // a word that holds the number of the last scatter with an amount that is not
+    // finite, and the running number
+    DevBuf splat_special;
+    uint32_t scatter_call = 0;
     std::array<int64_t, 4> src_cells{-1, -1, -1, -1};
     std::array<int, 4> src_classes{};
     int64_t dense_cap = 0, work_cap = 0, multi_cap = 0, part_acc_cap = 0;

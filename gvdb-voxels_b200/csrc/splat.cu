@@ -246,6 +246,9 @@ struct SplatArgs {
     // host does not know; all but the last class)
     const uint8_t *cell_cls;
     const int32_t *owner_list, *light_list;
+    // holds `call` when an amount of this call is not finite
+    uint32_t *special;
+    uint32_t call;
     int64_t owners;
 };
 
@@ -1836,7 +1839,9 @@ __device__ __forceinline__ void scatter_cell(const SplatArgs &S, ScChunk &C, int
     }
 }
 
-// kScWarps listed cells per CTA, a warp per cell.
+// kScWarps listed cells per CTA, a warp per cell.  Where some amount of the call is
+// not finite they take the light form too: the general one multiplies amounts by the
+// zero weights of rows and columns beyond a stencil.
 template <int KERNEL, int NCH>
 __global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_cells(SplatArgs S) {
     extern __shared__ __align__(16) unsigned char sc_smem[];
@@ -1845,7 +1850,10 @@ __global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_cells(S
     if (i >= S.owners) return;
     const int64_t cell = S.owner_list[i];
     if (!in_range(S.lim, cell, S.ncell, 28)) return;
-    scatter_cell<KERNEL, NCH>(S, reinterpret_cast<ScChunk *>(sc_smem)[warp], cell, lane);
+    static_assert(sizeof(LightWarp<NCH>) <= sizeof(ScChunk) && sizeof(ScChunk) % 16 == 0, "either form's share");
+    ScChunk &C = reinterpret_cast<ScChunk *>(sc_smem)[warp];
+    if (*S.special != S.call) scatter_cell<KERNEL, NCH>(S, C, cell, lane);
+    else scatter_light_cell<KERNEL, NCH>(S, reinterpret_cast<LightWarp<NCH> &>(C), cell, lane);
 }
 
 // Both forms in one launch, for volumes of few cells, in the list's order: the longest
@@ -1868,7 +1876,7 @@ __global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_owner(S
     const int64_t cell = S.owner_list ? (int64_t)S.owner_list[i] : i;
     if (!in_range(S.lim, cell, S.ncell, 46)) return;
     unsigned char *mine = sc_smem + warp * share;
-    if (S.cell_cls[cell] < kSrcClasses - 1)
+    if (S.cell_cls[cell] < kSrcClasses - 1 && *S.special != S.call)
         scatter_cell<KERNEL, NCH>(S, *reinterpret_cast<ScChunk *>(mine), cell, lane);
     else
         scatter_light_cell<KERNEL, NCH>(S, *reinterpret_cast<LightWarp<NCH> *>(mine), cell, lane);
@@ -2485,7 +2493,9 @@ __global__ void k_pack_amounts(SplatArgs S) {
     float a4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int c = 0; c < NCH; c++) a4[c] = ((S.attr_mask >> c) & 1) ? wt * load_f1(S.attr[c], p) : wt;
-    S.bin_amt[j] = make_float4(a4[0], a4[1], a4[2], a4[3]);
+    const float4 am = make_float4(a4[0], a4[1], a4[2], a4[3]);
+    S.bin_amt[j] = am;
+    if (!all_finite(am)) *S.special = S.call;
 }
 
 // A buffer of `bytes` that starts out zero: zeroed whenever it is
@@ -2524,6 +2534,10 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     // the list's count sits in its last 16 bytes
     S.merge_cnt = reinterpret_cast<uint32_t *>(v->merge_list.as<char>() + v->merge_list.bytes - 16);
     S.merge_list = v->merge_list.as<int32_t>();
+    GV_TRY(ensure_zeroed(v, v->splat_special, sizeof(uint32_t)));
+    if (++v->scatter_call == 0) v->scatter_call = 1; // 0: no call
+    S.special = v->splat_special.as<uint32_t>();
+    S.call = v->scatter_call;
     S.owner_list = v->ordered ? v->cell_owner.as<int32_t>() : nullptr;
     S.cell_cls = v->cell_cls.as<uint8_t>();
     S.owners = v->src_cells[NCH - 1];
