@@ -1882,9 +1882,16 @@ __global__ void __launch_bounds__(32 * kScWarps, kScMinBlocks) k_scatter_owner(S
         scatter_light_cell<KERNEL, NCH>(S, *reinterpret_cast<LightWarp<NCH> *>(mine), cell, lane);
 }
 
+// Listed cells a CTA of k_scatter_merge where the list is as long as it can be
+// (27 per dense cell, or every cell).  Mostly it is far shorter, often empty, and
+// CTAs with nothing to do cost their start: with a CTA a cell 54 us became 18 in
+// three launches of 4M points of a dam break, 19.4 became 13.2 in two of 300K, and
+// the full list of the 16M-point step went 228 -> 224.
+constexpr int kMergeCells = 4;
+
 // Adds the dense cells' partials to the cells listed by the owner-computes pass
-// (those with a dense cell among their 27): a CTA per listed cell (CTAs
-// past the list's end return), a thread per interior voxel, which adds, in
+// (those with a dense cell among their 27): a CTA per kMergeCells cells of the
+// longest list, one after the other, a thread per interior voxel, which adds, in
 // the order of kMergeMap, the partials that cover the voxel to the sum the
 // owner-computes pass wrote -- or writes them, for a cell listed as ~cell
 // (no owner sources: its sum is 0, and 0 + x is x).
@@ -1892,13 +1899,13 @@ template <int KERNEL, int NCH>
 __global__ void __launch_bounds__(512) k_scatter_merge(SplatArgs S) {
     using X = ExtTile<KERNEL>;
     __shared__ int32_t ne[27]; // partial slot of the dense cell in each direction, or -1
-    const uint32_t li = blockIdx.x;
-    if (li >= *S.merge_cnt) return;
-    {
+    const uint32_t count = *S.merge_cnt;
+    for (uint32_t li = blockIdx.x; li < count; li += gridDim.x) {
+        if (li >= gridDim.x) __syncthreads(); // the cell before is done with ne
         const int32_t entry = S.merge_list[li];
         const bool overwrite = entry < 0; // no owner sum to add to
         const int64_t cell = overwrite ? ~entry : entry;
-        if (!in_range(S.lim, cell, S.ncell, 23)) return;
+        if (!in_range(S.lim, cell, S.ncell, 23)) continue; // the same for the whole CTA
         int64_t slot;
         int cx, cy, cz;
         cell_coords(cell, S.m, S.m3, slot, cx, cy, cz);
@@ -2582,7 +2589,8 @@ gvdb2_status scatter_group(Volume *v, const SplatArgs &S0) {
     }
     // a cell with a dense cell among its 27 neighbours: at most 27 per dense cell
     const int64_t merge_grid = std::min<int64_t>(S.ncell, 27 * v->dense_cap);
-    if (merge_grid > 0) k_scatter_merge<KERNEL, NCH><<<(unsigned)merge_grid, 512, 0, v->stream>>>(S);
+    if (merge_grid > 0)
+        k_scatter_merge<KERNEL, NCH><<<(unsigned)((merge_grid + kMergeCells - 1) / kMergeCells), 512, 0, v->stream>>>(S);
     GV_CUDA(v, cudaGetLastError());
     return GVDB2_OK;
 }
