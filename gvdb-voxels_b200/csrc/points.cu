@@ -151,8 +151,10 @@ constexpr int64_t kCellCountReadback = 1 << 16; // cells
 // points are listed in `rows`, and their items apart in row_work.  cls gets each
 // cell's class of sources (SrcEdges), blk[k * gridDim.x + b] how many of block b's
 // cells are in class k, cnt[kCntSrc + k] how many of all.  Cells of at most `light` (<=
-// kLightCell) points are light.  All of it depends on the cell and its neighbours
-// alone, so that a cloud of a batch gets what a volume of its own gets.
+// kLightCell) points are light.  All of it depends on the cell, its brick and their
+// neighbours alone, so that a cloud of a batch gets what a volume of its own gets;
+// only the call's choice between rows and fixed point (default mode) counts cells
+// of the whole batch.
 // reg_off holds each (cell, region) bin's first entry; off[c] = reg_off[27 c], each
 // cell's (c = ncell: the end), is written for the kernels that follow.
 __global__ void k_cell_list(const uint32_t *reg_off, uint32_t *off, int64_t ncell, int32_t *list, int32_t *light, int2 *tiles,
